@@ -13,13 +13,17 @@ OBJ_DIR = os.path.join(HERE, '_build')          # objects: kept out of the shipp
 LIB = os.path.join(OUT_DIR, 'libsrwl_b200.so')
 NVCC = os.environ.get('NVCC', '/usr/local/cuda/bin/nvcc')
 ARCH = ['-gencode', 'arch=compute_100a,code=sm_100a']
-SOURCES = ['kernels.cu'] + ['line2_%d.cu' % l for l in range(6, 15)] + ['line2e_%d.cu' % l for l in range(6, 15)] + ['planner.cpp', 'tables.cpp', 'capi.cpp', 'noalloc.cu', 'lineg.cu', 'lineg_e.cu', 'multie.cu', 'mlp.cu', 'moments.cu', 'intensity.cu', 'gaussian.cu']
+SOURCES = ['kernels.cu', 'line2_14.cu', 'line2e_14.cu', 'planner.cpp', 'tables.cpp', 'capi.cpp', 'noalloc.cu',
+           'multie.cu', 'mlp.cu', 'moments.cu', 'intensity.cu', 'gaussian.cu']
+# the line passes on pairs: a unit per (axis, mode) (csrc/linep.cu)
+LINEP = ['linep.cu@%d,%d' % (c, m) for c in (0, 1) for m in (0, 1, 2)]
 
-def linen_lengths():
-    """Lengths of the specialised general-length line kernels (csrc/linen_lengths.h)."""
+
+def fixed_lengths():
+    """Lengths whose line pass has a fixed schedule, a unit each (csrc/linep_lengths.h)."""
     import re
-    txt = open(os.path.join(CSRC, 'linen_lengths.h')).read()
-    return sorted(set(int(v) for v in re.findall(r'X\((\d+)\)', txt)))
+    txt = open(os.path.join(CSRC, 'linep_lengths.h')).read()
+    return sorted((int(v) for v in re.findall(r'X\((\d+),', txt)), reverse=True)
 
 
 # host code: no FP contraction so the mesh bookkeeping rounds exactly like the reference
@@ -49,17 +53,21 @@ def _includes(path, seen):
 
 def _compile(s, ptxas_info):
     defs = []
-    if '@' in s:                      # linen.cu@N: the specialised general-length pass for N points
+    if '@' in s:
         s, n = s.split('@')
-        defs = ['-DSRWG_LINEN=' + n]
-        obj = os.path.join(OBJ_DIR, 'linen_%s.cu.o' % n)
+        if ',' in n:
+            c, m = n.split(',')
+            defs = ['-DSRWG_LINEP_COLS=' + c, '-DSRWG_LINEP=' + m]
+        else:
+            defs = ['-DSRWG_LINEF_N=' + n]
+        obj = os.path.join(OBJ_DIR, 'linep_%s.cu.o' % n.replace(',', '_'))
     else:
         obj = os.path.join(OBJ_DIR, s + '.o')
     src = os.path.join(CSRC, s)
     deps = sorted(_includes(src, set()))
     if os.path.exists(obj) and os.path.getmtime(obj) >= max(os.path.getmtime(d) for d in deps) and not ptxas_info:
         return obj, ''
-    cmd = [NVCC, '-c', '-O3', '-std=c++17', '-lineinfo', '-Xcompiler', HOST_FLAGS, '--fmad=true'] + ARCH + \
+    cmd = [NVCC, '-c', '-O3', '-std=c++17', '-lineinfo', '-Xcompiler', HOST_FLAGS, '--fmad=true', '-Xfatbin=-compress-all'] + ARCH + \
           defs + ['-I', CSRC, '-o', obj, src]
     if ptxas_info and s.endswith('.cu'):
         cmd.insert(1, '-Xptxas=-v')
@@ -70,9 +78,7 @@ def build(verbose=False, ptxas_info=False):
     from concurrent.futures import ThreadPoolExecutor
     os.makedirs(OUT_DIR, exist_ok=True)
     os.makedirs(OBJ_DIR, exist_ok=True)
-    units = SOURCES + ['linen.cu@%d' % n for n in linen_lengths()]
-    # longest units first, so that the pool's last wave is short
-    units.sort(key=lambda u: (not u.startswith('line2'), u))
+    units = LINEP + ['linep.cu@%d' % n for n in fixed_lengths()] + SOURCES          # longest units first
     with ThreadPoolExecutor(max_workers=max(1, min(len(units), os.cpu_count() or 1))) as ex:
         res = list(ex.map(lambda s: _compile(s, ptxas_info), units))
     objs = [o for o, _ in res]

@@ -18,6 +18,7 @@
 #include "errors.h"
 #include "kernels.h"
 #include "exec.h"
+#include "linep_shape.h"
 #include "planner.h"
 
 namespace srwg {
@@ -71,46 +72,49 @@ int device_ctx(int dev, DeviceCtx** out)
     return 0;
 }
 
-// exp(-2 pi i k/N) in FP64, rounded to FP32
+static std::mutex g_shapeMutex;
+static std::map<int, PairShape> g_shapes;
+static const PairShape* pair_shape(int N)
+{
+    std::lock_guard<std::mutex> lk(g_shapeMutex);
+    auto it = g_shapes.find(N);
+    if (it == g_shapes.end()) {
+        PairShape z;
+        if (!make_pair_shape(N, z)) z.n = 0;
+        it = g_shapes.emplace(N, z).first;
+    }
+    return it->second.n ? &it->second : nullptr;
+}
+
+bool pair_supported(int N) { return pair_shape(N) != nullptr; }
+
+// passes on pairs: the stages' tables (linep_shape.h); 16384 points: exp(-2 pi i k / N)
+void line_twiddles(int N, std::vector<float2>& h)
+{
+    const PairShape* z = pair_shape(N);
+    if (z != nullptr) {
+        fill_twiddles(*z, h);
+        return;
+    }
+    h.resize(N);
+    for (int k = 0; k < N; k++) {
+        const double a = -2. * M_PI * (double)k / (double)N;
+        h[k] = make_float2((float)cos(a), (float)sin(a));
+    }
+}
+
 int device_twiddles(DeviceCtx& c, int N, const float2** out)
 {
     auto it = c.tw.find(N);
     if (it != c.tw.end()) { *out = it->second; return 0; }
-    std::vector<float2> h(N);
-    for (int k = 0; k < N; k++) {
-        double a = -2. * M_PI * (double)k / (double)N;
-        h[k] = make_float2((float)cos(a), (float)sin(a));
-    }
+    std::vector<float2> h;
+    line_twiddles(N, h);
     float2* d = nullptr;
-    CUDA_TRY(cudaMalloc(&d, sizeof(float2) * N));
-    CUDA_TRY(cudaMemcpy(d, h.data(), sizeof(float2) * N, cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMalloc(&d, sizeof(float2) * h.size()));
+    CUDA_TRY(cudaMemcpy(d, h.data(), sizeof(float2) * h.size(), cudaMemcpyHostToDevice));
     c.tw[N] = d;
     *out = d;
     return 0;
-}
-
-// radix schedule of an even N: power-of-two part in radix-16/8 stages (4/8-bit splits), then 3, 5, 7, 11, 13
-int radix_plan(int N, int* r)
-{
-    int n = N, p2 = 0, ns = 0;
-    while (n % 2 == 0) { n /= 2; p2++; }
-    int odd[32], no = 0;
-    const int primes[5] = {3, 5, 7, 11, 13};
-    for (int i = 0; i < 5; i++)
-        while (n % primes[i] == 0) { odd[no++] = primes[i]; n /= primes[i]; }
-    if (n != 1) return -1;
-    int bits[16], nb = 0;
-    while (p2 >= 4 && p2 != 5) {
-        if (p2 == 6) { bits[nb++] = 3; bits[nb++] = 3; p2 = 0; break; }
-        bits[nb++] = 4;
-        p2 -= 4;
-    }
-    if (p2 == 5) { bits[nb++] = 3; bits[nb++] = 2; p2 = 0; }
-    else if (p2 >= 1 && p2 <= 3) { bits[nb++] = p2; p2 = 0; }
-    for (int i = 0; i < nb; i++) r[ns++] = 1 << bits[i];
-    for (int i = 0; i < no; i++) r[ns++] = odd[i];
-    if (ns > SRWG_MAX_STAGES) return -1;
-    return ns;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -200,103 +204,74 @@ int fixed_lines_per_cta(int axis, int N)
     return fam == FAM_POW2 ? line2_lines_per_cta(axis, N) : linen_lines_per_cta(axis, N);
 }
 
+// pairs of lines per CTA: the tuned lines halved, else about 256 threads (columns: at least two pairs,
+// 32-byte pieces of a row, a power of two)
+static int pairs_per_cta(int axis, int N, const PairShape& z)
+{
+    const int lines = tuned(axis, N).lines;
+    int G = lines > 0 ? lines / 2 : 256 / z.T;
+    if (axis == 1 && lines == 0 && G < 2) G = 2;
+    if (G < 1) G = 1;
+    if (axis == 1) {
+        if (G > 16) G = 16;
+        while (G & (G - 1)) G &= G - 1;
+    }
+    while (G > 1 && (G * z.T > 512 || (size_t)G * (z.slot + 8) * 16 > SRWG_LINE_SMEM_MAX)) G = axis == 1 ? G / 2 : G - 1;
+    return G;
+}
+
+int pair_block(int N, int nl)
+{
+    const PairShape* z = pair_shape(N);
+    if (z == nullptr) return 0;
+    int w = 2 * pairs_per_cta(1, N, *z);
+    if (w < 4) w = 4;                        // whole 32-byte sectors for the row pass
+    return nl % w == 0 ? w : 0;
+}
+
 int line_config(const LineDesc& d, LineLaunch& p)
 {
     p.d = d;
-    int N = d.axis == 0 ? d.nx : d.nz;
+    const int N = d.axis == 0 ? d.nx : d.nz;
     p.N = N;
     p.nlines = d.axis == 0 ? d.nz : d.nx;
-    const size_t cap = SRWG_LINE_SMEM_MAX;
-    const int fam = fixed_family(d.axis, N);
-    if (fam == FAM_POW2) {
-        // power of two: 16 points per thread, radix-16 stages then a 16/8/4/2 stage
+    const PairShape* z = pair_shape(N);
+    if (z != nullptr) {
+        p.v2 = 0;
+        p.T = z->T;
+        p.G = pairs_per_cta(d.axis, N, *z);
+        p.nst = z->n;
+        for (int s = 0; s < z->n; s++) { p.radix[s] = z->R[s]; p.dR[s] = z->dR[s]; p.dB[s] = z->dB[s]; p.tw1[s] = z->tw1[s]; p.tw2[s] = z->tw2[s]; }
+        for (int s = 0; s <= z->n; s++) { p.len[s] = z->len[s]; p.dL[s] = z->dL[s]; }
+        p.pitch = z->pitch;
+        // a windowed row pass on blocks of rows takes whole blocks where they are small
+        if (d.axis == 0 && d.zwin && d.blk_in > 0) {
+            const int G = d.blk_in / 2;
+            if (!d.out_int && G * z->T <= 256) p.G = G;
+        }
+        if (d.axis == 0 && d.out_int) p.G = std::max(1, 128 / z->T);
+        // few lines: rather more CTAs than pairs sharing one
+        if (d.axis == 0)
+            while (p.G > 1 && (long long)p.nlines * std::max(1, p.nb) < 148LL * 2 * p.G) p.G = (p.G + 1) / 2;
+        p.L = (d.out_int ? 1 : 2) * p.G;
+        // slots of a column tile start 8 / G places apart (their pairs read neighbouring lines together)
+        p.P = z->slot;
+        if (d.axis == 1 && p.G >= 2) {
+            const int r = p.G >= 8 ? 1 : 8 / p.G;
+            p.P += (r + 8 - p.P % 8) % 8;
+        }
+        return 0;
+    }
+    if (N == 16384) {
+        // 16 points of one line per thread, radix-16 stages (line2.cuh)
         p.v2 = 1;
         p.T = N / 16;
-        int nb = 0;
-        while ((1 << nb) < N) nb++;
-        p.nst = 0;
-        while (nb > 4 && nb - 4 >= 1) {
-            if (nb - 4 < 1) break;
-            p.radix[p.nst++] = 16;
-            nb -= 4;
-        }
-        p.radix[p.nst++] = 1 << nb;          // 16, 8, 4 or 2
-        const int L = fixed_lines_per_cta(d.axis, N);
-        p.P = (int)line_pitch(N, L, d.axis == 1);
-        if (p.T * L > 1024) { g_lastDetail = "line pass too large"; return SRWG_ERR_UNSUPPORTED; }
-        p.L = L;
-        p.G = L;
-        if ((size_t)p.L * p.P * sizeof(float2) > cap) { g_lastDetail = "line too long for shared memory"; return SRWG_ERR_UNSUPPORTED; }
+        p.L = p.G = 1;
+        p.P = (int)line_pitch(N, 1, d.axis == 1);
         return 0;
     }
-    // general length (or a power of two the tuner gave it) with a specialised kernel (linen.cuh):
-    // compile-time schedule, T = ceil(N/16)
-    if (fam == FAM_SPEC) {
-        p.v2 = 3;
-        p.T = (N + 15) / 16;
-        p.L = fixed_lines_per_cta(d.axis, N);
-        p.P = (int)line_pitch(N, p.L, d.axis == 1);
-        p.G = p.L;
-        p.nst = 0;
-        if (p.T * p.L > 512 || (size_t)p.L * p.P * sizeof(float2) > cap) {
-            g_lastDetail = "line too long for shared memory";
-            return SRWG_ERR_UNSUPPORTED;
-        }
-        return 0;
-    }
-    // general good number with radices 16/8/4/2, 3, 5, 7 and at least two stages: the fused pass of
-    // lineg.cuh (T >= N/16 threads per line, rows ~256 threads, columns up to 512 threads per CTA)
-    {
-        int rad[SRWG_MAX_STAGES];
-        const int ns = radix_plan(N, rad);
-        bool gen = ns >= 2 && N <= 8192;
-        for (int i = 0; i < ns && gen; i++) gen = rad[i] != 11 && rad[i] != 13;
-        if (gen) {
-            p.v2 = 2;
-            int T = (N + 15) / 16;
-            T = ((T + 31) / 32) * 32;
-            p.T = T;
-            int L = d.axis == 0 ? 256 / T : 512 / T;
-            if (L < 1) L = 1;
-            while (L > 1 && (size_t)L * line_pitch(N, L, d.axis == 1) * sizeof(float2) > cap) L--;
-            p.P = (int)line_pitch(N, L, d.axis == 1);
-            if (T * L > 512 || (size_t)L * p.P * sizeof(float2) > cap) {
-                g_lastDetail = "line too long for shared memory";
-                return SRWG_ERR_UNSUPPORTED;
-            }
-            p.L = L;
-            p.G = L;
-            p.nst = ns;
-            for (int i = 0; i < ns; i++) p.radix[i] = rad[i];
-            return 0;
-        }
-    }
-    p.v2 = 0;
-    // general good number: T threads per line, at most 16 points each; G = threads per CTA / T
-    // groups work on the CTA's L lines in batches
-    int T = (N + 15) / 16;
-    T = ((T + 31) / 32) * 32;
-    if (T < 32) T = 32;
-    if (T > 512) { g_lastDetail = "FFT length above 8192"; return SRWG_ERR_UNSUPPORTED; }
-    p.T = T;
-    int L;
-    if (d.axis == 0) {
-        L = 256 / T > 1 ? 256 / T : 1;          // rows: ~256 threads, one batch
-        p.P = N;
-    } else {
-        L = 512 / T > 4 ? 512 / T : 4;          // columns: >= 4 per tile (32-byte row segments)
-        p.P = N + 1;
-    }
-    while (L > 1 && (size_t)L * p.P * sizeof(float2) > cap) L--;
-    p.L = L;
-    if ((size_t)p.L * p.P * sizeof(float2) > cap) { g_lastDetail = "line too long for shared memory"; return SRWG_ERR_UNSUPPORTED; }
-    int G = 512 / T;
-    if (G > L) G = L;
-    if (G < 1) G = 1;
-    p.G = G;
-    p.nst = radix_plan(N, p.radix);
-    if (p.nst < 0) { g_lastDetail = "FFT length is not 2^a 3^b 5^c 7^d 11^e 13^f"; return SRWG_ERR_UNSUPPORTED; }
-    return 0;
+    g_lastDetail = N > 8192 ? "FFT length above 8192" : "FFT length is not 2^a 3^b 5^c 7^d 11^e 13^f";
+    return SRWG_ERR_UNSUPPORTED;
 }
 
 // device copy of a plan's constant data: its point-wise tables, then (256-byte aligned) its pass
@@ -387,6 +362,8 @@ int execute_passes(const std::vector<KernelDesc>& ks, DeviceCtx& c, int nb, cons
         float2* d1 = toOut ? outY : wb[k.dst][1];
         const long long bSrc = fromOut ? outStride : fromIn ? inStride : (long long)workElems;
         const long long bDst = toOut ? outStride : (long long)workElems;
+        // line passes may be set up while the pass before them ends (not between timing events)
+        const bool pdlOk = i > 0 && ev == nullptr;
         cudaError_t e = cudaSuccess;
         if (k.kind == K_MOM) {
             if (momScratch == nullptr || momSlots == nullptr || k.mom.slot < 0 || k.mom.slot >= nSlots) {
@@ -415,6 +392,7 @@ int execute_passes(const std::vector<KernelDesc>& ks, DeviceCtx& c, int nb, cons
         } else if (k.kind == K_LINE) {
             LineLaunch p;
             memset(&p, 0, sizeof(p));
+            p.nb = nb;
             int r = line_config(k.line, p);
             if (r) return r;
             r = device_twiddles(c, p.N, &p.tw);
@@ -425,8 +403,10 @@ int execute_passes(const std::vector<KernelDesc>& ks, DeviceCtx& c, int nb, cons
             p.nb = nb; p.bDesc = constStride; p.bTab = tabStride; p.bSrc = bSrc; p.bDst = bDst;
             p.status = c.status;
             p.spin = g_waitLimit;
+            p.byValue = hostMax == nullptr;
+            p.run = k.line.run;
             line_window(k.line, p);
-            e = launch_line(p, st);
+            e = launch_line(p, st, pdlOk);
         } else if (k.kind == K_RESIZE) {
             ResizeLaunch p;
             memset(&p, 0, sizeof(p));
@@ -503,6 +483,7 @@ static int execute(Planner& pl, DeviceCtx& c, const float2* inX, const float2* i
 
 static int ensure_work(DeviceCtx& c, size_t elems)
 {
+    elems += elems & 1;                          // 16-byte aligned fields
     if (c.workElems >= elems && c.work) return 0;
     if (c.work) { cudaFree(c.work); c.work = nullptr; c.workElems = 0; }
     CUDA_TRY(cudaMalloc(&c.work, 4 * elems * sizeof(float2)));
@@ -939,7 +920,7 @@ int srwgPlanExecuteBatch(srwgPlan* plan, int n, const float* dExIn, const float*
     DeviceCtx& c = *plan->ctx;
     if ((strideIn & 1) || (strideOut & 1)) return SRWG_ERR_BAD_ARG;     // whole complex points
     // one launch per pass for the whole batch (grid z = wavefront) when the work buffers hold it
-    const size_t per = (size_t)plan->pl.maxElems;
+    const size_t per = ((size_t)plan->pl.maxElems + 1) & ~(size_t)1;     // 16-byte aligned fields
     int chunk = n;
     const size_t budget = (size_t)1 << 30;                               // work elements (8 GiB)
     while (chunk > 1 && 4 * (size_t)chunk * per > budget) chunk = (chunk + 1) / 2;

@@ -7,6 +7,12 @@
 
 namespace srwg {
 
+// programmatic dependent launch: the next kernel in the stream may be set up from here on; this one
+// waits until the kernel before it has completed and its writes are visible.  (Both do nothing in an
+// ordinary launch.)
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ float2 cmul(float2 a, float2 b)
 {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);

@@ -16,7 +16,7 @@
 #include <stdint.h>
 
 #define SRWG_MAX_MASKS 4
-#define SRWG_MAX_STAGES 12
+#define SRWG_MAX_STAGES 8
 #define SRWG_MAX_KERNELS 64
 
 // Aperture / obstacle mask in physical coordinates (sroptapt.h:118-395).  The physical coordinate
@@ -74,10 +74,32 @@ struct FftSide {
     float scale;         // real factor (1 if none)
 };
 
+// What a line pass on pairs reads of its descriptor (filled from it, fill_line_run): offsets are in
+// float2 units into the plan's tables, -1 when absent.
+struct alignas(16) LineRun {
+    int dir1, dir2;                 // directions of the transforms (+1, -1; dir1 0: the single one is the second)
+    int pre_rot, mid_in, mid_mir, mid_out, fin_rot;   // centring rotations and mirror of the chains
+    int pre_tab, mid_tab, fin_tab;  // factors along the line
+    int lt[3];                      // line factors (pre, mid, fin; the absent ones last)
+    int mirror_lines;
+    int zwin, zl0, zl1, za0, za1, zskip;
+    int blk_in, blk_out;
+    int extra;                      // the middle chain has non-separable work
+    int int_flat;
+    float int_scale;
+    int ang;                        // quartic part of the angular transfer function in the middle chain (two
+    int qtab, qline;                //   transforms): 0 none, 1 |phase| < 0.03, 2 any; tables of q^2 (floats)
+    float qc0, qc1;                 //   along the line and per line, phase = qc0 q2 (qc1 q2)(1 + 2 qc1 q2)
+    int pad[2];
+};
+
 struct LineDesc {
+    LineRun run;
     int axis;            // 0: rows (transform along x), 1: columns (transform along z)
     int nx, nz;
     int f1;              // 0 none, +1 forward, -1 inverse: first transform along the line
+    int dir1;            // its direction as it runs: -f1 where a mirror between two transforms is folded
+                         //   into the first one (tables.cpp), else f1
     FftSide f1_pre, f1_post;
     int has_pw;
     PwOps pw;
@@ -99,6 +121,8 @@ struct LineDesc {
     int out_int;                    // last pass of a multi-electron batch on a specialised kernel: one
                                     //   CTA transforms both components of its lines and writes the
                                     //   total intensity |Ex|^2 + |Ey|^2 (float, dst[0]) instead of them
+    int ang, qtab, qline;           // see LineRun
+    float qc0, qc1;
     int int_flat;                   // intensity pass whose output factors (the output chain's table,
     float int_scale;                //   the line factors) have one magnitude everywhere: they are not
                                     //   applied, the intensity is scaled by int_scale = that magnitude^2

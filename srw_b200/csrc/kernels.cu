@@ -5,6 +5,7 @@
 // no tensor cores.  Phase arguments are formed and reduced modulo 2*pi in FP64 and evaluated
 // with an FP32 sincosf, as the reference forms them in double before its float CosAndSin
 // (sroptelm.h:856-871).
+#include <algorithm>
 #include <mutex>
 #include <set>
 
@@ -22,110 +23,6 @@ static bool attrs_needed(int group)
     if (cudaGetDevice(&dev) != cudaSuccess) return true;
     std::lock_guard<std::mutex> lk(m);
     return done.insert(((long long)dev << 8) | group).second;
-}
-
-// ------------------------------------------------------------------------------------------------
-// LINE pass: a CTA owns L whole rows (axis 0) or L whole columns (axis 1) in shared memory; G
-// thread groups of T threads transform them in ceil(L/G) batches (T*G <= 512 threads, so each
-// thread can hold its 16 in-flight points and twiddles in registers).
-// ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(512, 1) line_kernel(const LineLaunch p)
-{
-    extern __shared__ float2 sm[];
-    // descriptor in shared memory: point-wise code takes references to it (a reference to a
-    // kernel parameter would force a copy of the whole parameter block to local memory)
-    const LineDesc& d = *reinterpret_cast<const LineDesc*>(reinterpret_cast<const char*>(p.gd) + blockIdx.z * p.bDesc);
-    __shared__ int radix[SRWG_MAX_STAGES];
-    if (threadIdx.x < SRWG_MAX_STAGES) radix[threadIdx.x] = p.radix[threadIdx.x];
-    __syncthreads();
-    const int comp = blockIdx.y;
-    const float2* __restrict__ src = p.src[comp] + blockIdx.z * p.bSrc;
-    float2* __restrict__ dst = p.dst[comp] + blockIdx.z * p.bDst;
-    const int N = p.N, T = p.T, L = p.L, P = p.P, nl = p.nlines;
-    const int tid = threadIdx.x, nth = blockDim.x;
-    const int G = nth / T;
-    const int g = tid / T, t = tid - g * T;
-    const int line0 = (blockIdx.x + p.blk0) * L;
-
-    // ---- load the tile
-    if (d.axis == 0) {
-        for (int e = tid; e < N * L; e += nth) {
-            int c = e / N, k = e - c * N;
-            if (line0 + c < nl) sm[(size_t)c * P + k] = __ldcs(&src[(size_t)(line0 + c) * N + k]);
-        }
-    } else {
-        for (int e = tid; e < N * L; e += nth) {
-            int r = e / L, c = e - r * L;
-            int col = line0 + c;
-            if (col < nl) sm[(size_t)c * P + r] = __ldcs(&src[(size_t)r * nl + col]);
-        }
-    }
-    __syncthreads();
-
-    // chains with their along-line factors in the plan's tables (as the power-of-two kernels); the
-    // per-line factors of all chains are multiplied once and applied at the store
-    const float2* tabs = p.tabs + blockIdx.z * p.bTab;
-    const PwOps* ex = &d.extra;
-    ChainG pre, mid, fin;
-    pre.rs1 = 0; pre.mir = 0; pre.rs2 = d.f1_pre.rs; pre.tab = (int)d.t_pre.tab; pre.extra = 0;
-    mid.rs1 = d.f1 ? d.f1_post.rs : 0; mid.mir = d.mirror_along; mid.rs2 = d.f2 ? d.f2_pre.rs : 0;
-    mid.tab = (int)d.t_mid.tab; mid.extra = d.has_extra;
-    if (d.f2) {
-        fin.rs1 = d.f2_post.rs; fin.mir = 0; fin.rs2 = 0; fin.tab = (int)d.t_fin.tab; fin.extra = 0;
-    } else {
-        fin = mid;
-    }
-    const bool has_lf = (d.t_pre.ltab >= 0) || (d.t_mid.ltab >= 0) || (d.t_fin.ltab >= 0);
-
-    // ---- transforms, batch by batch (uniform trip count: every thread reaches every barrier)
-    if (d.f1 || d.f2) {
-        const int nb = (L + G - 1) / G;
-        for (int it = 0; it < nb; it++) {
-            const int c = it * G + g;
-            const int line = line0 + c;
-            const bool active = (g < G) && (c < L) && (line < nl);
-            float2* s = sm + (size_t)(c < L ? c : 0) * P;
-            if (d.f1) {
-                if (!chainG_trivial(pre)) gather_pass_t(s, N, line, pre, t, T, active, tabs, ex, d.axis);
-                if (d.f1 > 0) run_fft<1>(s, N, radix, p.nst, p.tw, t, T, active);
-                else run_fft<-1>(s, N, radix, p.nst, p.tw, t, T, active);
-            }
-            if (d.f2) {
-                if (!chainG_trivial(mid)) gather_pass_t(s, N, line, mid, t, T, active, tabs, ex, d.axis);
-                if (d.f2 > 0) run_fft<1>(s, N, radix, p.nst, p.tw, t, T, active);
-                else run_fft<-1>(s, N, radix, p.nst, p.tw, t, T, active);
-            }
-        }
-    }
-    const bool triv = chainG_trivial(fin) && !has_lf;
-
-    // ---- store the tile
-    for (int e = tid; e < N * L; e += nth) {
-        int c, k;
-        if (d.axis == 0) { c = e / N; k = e - c * N; }
-        else { k = e / L; c = e - k * L; }
-        const int line = line0 + c;
-        if (line >= nl) continue;
-        const float2* sc = sm + (size_t)c * P;
-        float2 v;
-        if (triv) {
-            v = sc[k];
-        } else {
-            int i;
-            const int sr = chainG_src(fin, k, N, i);
-            v = cmul(chainG_factor(fin, k, i, line, tabs, ex, d.axis), sc[sr]);
-            if (has_lf) {
-                float2 lf = make_float2(1.f, 0.f);
-                if (d.t_pre.ltab >= 0) lf = cmul(lf, __ldg(&tabs[d.t_pre.ltab + line]));
-                if (d.t_mid.ltab >= 0) lf = cmul(lf, __ldg(&tabs[d.t_mid.ltab + line]));
-                if (d.t_fin.ltab >= 0) lf = cmul(lf, __ldg(&tabs[d.t_fin.ltab + line]));
-                v = cmul(lf, v);
-            }
-        }
-        const int ol = d.mirror_lines ? (nl - 1 - line) : line;
-        if (d.axis == 0) __stcs(&dst[(size_t)ol * N + k], v);
-        else __stcs(&dst[(size_t)k * nl + ol], v);
-    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -584,34 +481,46 @@ __global__ void __launch_bounds__(256) pw_kernel(const PwLaunch p)
 // ------------------------------------------------------------------------------------------------
 // launchers
 // ------------------------------------------------------------------------------------------------
-Line2Fn line2_kernel_ptr(int logn, bool cols, bool extra, int f1, int f2)
+// the line pass of N points: the fixed schedule where the length has one
+static LineFn line_fn(int N, bool cols, int mode, int extra)
 {
-    switch (logn) {
-    case 6: return extra ? line2e_get_6(cols, f1, f2) : line2_get_6(cols, f1, f2);
-    case 7: return extra ? line2e_get_7(cols, f1, f2) : line2_get_7(cols, f1, f2);
-    case 8: return extra ? line2e_get_8(cols, f1, f2) : line2_get_8(cols, f1, f2);
-    case 9: return extra ? line2e_get_9(cols, f1, f2) : line2_get_9(cols, f1, f2);
-    case 10: return extra ? line2e_get_10(cols, f1, f2) : line2_get_10(cols, f1, f2);
-    case 11: return extra ? line2e_get_11(cols, f1, f2) : line2_get_11(cols, f1, f2);
-    case 12: return extra ? line2e_get_12(cols, f1, f2) : line2_get_12(cols, f1, f2);
-    case 13: return extra ? line2e_get_13(cols, f1, f2) : line2_get_13(cols, f1, f2);
-    case 14: return extra ? line2e_get_14(cols, f1, f2) : line2_get_14(cols, f1, f2);
-    default: return nullptr;
+    switch (N) {
+#define SRWG_LINEF_CASE(M, A, B, C, D, T) case M: return linef_get_##M(cols, mode, extra);
+    SRWG_LINEF_LENGTHS(SRWG_LINEF_CASE)
+#undef SRWG_LINEF_CASE
+    default: break;
+    }
+    switch (mode + (cols ? 3 : 0)) {
+    case 0: return linep_get_0_0(extra);
+    case 1: return linep_get_0_1(extra);
+    case 2: return linep_get_0_2(extra);
+    case 3: return linep_get_1_0(extra);
+    case 4: return linep_get_1_1(extra);
+    default: return linep_get_1_2(extra);
     }
 }
 
-Line2Fn linen_kernel_ptr(int N, bool cols, bool extra, int nt, bool inten)
+// launches f; pdl: as a programmatic dependent of the kernel before it in the stream
+template <class A>
+static cudaError_t launch_one(void (*f)(const A), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, const A& a)
 {
-#define SRWG_LINEN_CASE(M) if (N == M) return linen_get_##M(cols, extra, nt, inten);
-    SRWG_LINEN_LENGTHS(SRWG_LINEN_CASE)
-    SRWG_LINEN_POW2(SRWG_LINEN_CASE)
-#undef SRWG_LINEN_CASE
-    return nullptr;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, f, a);
 }
 
-cudaError_t launch_line(const LineLaunch& pin, cudaStream_t st)
+cudaError_t launch_line(const LineLaunch& pin, cudaStream_t st, bool pdl)
 {
-    LineLaunch p = pin;
+    LineArgs p = pin;
+    const LineDesc& d = pin.d;
     dim3 grid((p.nlines + p.L - 1) / p.L, 2, p.nb > 1 ? p.nb : 1);
     if (p.nblk > 0) {
         // only the line blocks of the window (the others would write nothing)
@@ -620,59 +529,59 @@ cudaError_t launch_line(const LineLaunch& pin, cudaStream_t st)
     } else {
         p.blk0 = 0;
     }
-    size_t smem = (size_t)p.L * p.P * sizeof(float2);
-    if (smem > SRWG_LINE_SMEM_MAX) return cudaErrorInvalidValue;
     if (attrs_needed(0)) {
-        cudaFuncSetAttribute(line_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SRWG_LINE_SMEM_MAX);
         const int dirs[8][2] = {{1, 1}, {1, -1}, {-1, 1}, {-1, -1}, {1, 0}, {-1, 0}, {0, 1}, {0, -1}};
-        for (int lg = 6; lg <= 14; lg++)
-            for (int e = 0; e < 4; e++)
-                for (int m = 0; m < 8; m++)
-                    cudaFuncSetAttribute(line2_kernel_ptr(lg, e & 1, e >> 1, dirs[m][0], dirs[m][1]),
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, SRWG_LINE_SMEM_MAX);
         for (int e = 0; e < 2; e++) {
-            cudaFuncSetAttribute(lineg_get(e != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, SRWG_LINE_SMEM_MAX);
-            cudaFuncSetAttribute(lineg_e_get(e != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, SRWG_LINE_SMEM_MAX);
+            for (int m = 0; m < 8; m++) {
+                cudaFuncSetAttribute(line2_get_14(e, dirs[m][0], dirs[m][1]),
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, SRWG_LINE_SMEM_MAX);
+                cudaFuncSetAttribute(line2e_get_14(e, dirs[m][0], dirs[m][1]),
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, SRWG_LINE_SMEM_MAX);
+            }
+            const int modes[6][2] = {{0, 0}, {0, 2}, {1, 0}, {1, 1}, {1, 2}, {2, 0}};
+            for (const auto& m : modes) {
+                cudaFuncSetAttribute(line_fn(0, e, m[0], m[1]), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     SRWG_LINE_SMEM_MAX);
+#define SRWG_LINEF_ATTR(M, A, B, C, D, T)                                                                   \
+                cudaFuncSetAttribute(line_fn(M, e, m[0], m[1]), cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                     SRWG_LINE_SMEM_MAX);
+                SRWG_LINEF_LENGTHS(SRWG_LINEF_ATTR)
+#undef SRWG_LINEF_ATTR
+            }
         }
-#define SRWG_LINEN_ATTR(M)                                                                                 \
-        for (int e = 0; e < 10; e++)                                                                       \
-            cudaFuncSetAttribute(linen_get_##M(e & 1, (e >> 1) & 1, 1 + ((e >> 2) & 1), e >= 8),           \
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, SRWG_LINE_SMEM_MAX);
-        SRWG_LINEN_LENGTHS(SRWG_LINEN_ATTR)
-        SRWG_LINEN_POW2(SRWG_LINEN_ATTR)
-#undef SRWG_LINEN_ATTR
     }
-    if (p.d.out_int && p.v2 != 3) return cudaErrorInvalidValue;    // intensity passes: specialised kernels only
-    if (p.v2 == 3) {
-        const bool inten = p.d.out_int != 0;
-        if (inten && (p.d.has_extra || (p.d.f1 && p.d.f2))) return cudaErrorInvalidValue;
-        Line2Fn f = linen_kernel_ptr(p.N, p.d.axis != 0, p.d.has_extra != 0, (p.d.f1 && p.d.f2) ? 2 : 1, inten);
-        if (f == nullptr || p.T * p.L > 512) return cudaErrorInvalidValue;
-        if (inten) {
-            grid.y = 1;                         // one CTA transforms both components of its lines
-            // the first component's intensity of every point a thread stores, in shared memory
-            // after the line slots
-            smem += (size_t)linen_int_floats(p.N) * p.T * p.L * sizeof(float);
-            if (smem > SRWG_LINE_SMEM_MAX) return cudaErrorInvalidValue;
+    if (p.v2 == 0) {
+        const bool inten = d.out_int != 0;
+        if (inten && (d.has_extra || (d.f1 && d.f2))) return cudaErrorInvalidValue;
+        size_t smem = (size_t)p.G * p.P * sizeof(float4);
+        // a windowed tile that is one block of its input (the pass before it wrote blocks of this width):
+        // the window by bulk copies into shared memory behind the slots, where that leaves the CTAs per SM
+        // (two of 256 threads at 128 registers, more of fewer) room.  The largest window of the launch
+        // is the host's; an electron's larger one loads directly.
+        p.bulk = 0;
+        if (d.zwin && d.blk_in == p.L && d.za0 <= d.za1 && ((((uintptr_t)p.src[0]) | ((uintptr_t)p.src[1])) & 15) == 0 &&
+            (p.bSrc & 1) == 0 && (p.L & 1) == 0) {
+            const size_t pts = (size_t)(std::min(p.N, d.za1 - d.za0 + 9)) * p.L;
+            const size_t stg = pts * sizeof(float2) * (inten ? 2 : 1);
+            const int ctas = std::min(4, std::max(1, 512 / (p.T * p.G)));
+            if ((smem + stg + 1024) * ctas <= SRWG_LINE_SMEM_MAX) {
+                p.bulk = (int)pts;
+                smem += stg;
+            }
         }
-        // input tiles by bulk async copies: 16-byte aligned sources; rows are contiguous, columns
-        // only when the row pass wrote them in blocks of exactly the tile's (even) width
-        LineLaunch q = p;
-        const bool aligned = ((((uintptr_t)p.src[0]) | ((uintptr_t)p.src[1])) & 15) == 0 && (p.bSrc & 1) == 0;
-        q.bulk = aligned && (p.d.axis == 0 || (p.d.blk_in == p.L && (p.L & 1) == 0));
-        f<<<grid, p.T * p.L, smem, st>>>(q);
-    } else if (p.v2 == 2) {
-        Line2Fn f = p.d.has_extra ? lineg_e_get(p.d.axis != 0) : lineg_get(p.d.axis != 0);
-        if (p.T * p.L > 512) return cudaErrorInvalidValue;
-        f<<<grid, p.T * p.L, smem, st>>>(p);
-    } else if (p.v2) {
-        int lg = 0;
-        while ((1 << lg) < p.N) lg++;
-        Line2Fn f = line2_kernel_ptr(lg, p.d.axis != 0, p.d.has_extra != 0, p.d.f1, p.d.f2);
+        if (p.T * p.G > 512 || smem > SRWG_LINE_SMEM_MAX || (!inten && (p.nlines & 1))) return cudaErrorInvalidValue;
+        p.alignIn = ((((uintptr_t)p.src[0]) | ((uintptr_t)p.src[1])) & 15) == 0 && (p.bSrc & 1) == 0;
+        p.alignOut = ((((uintptr_t)p.dst[0]) | ((uintptr_t)p.dst[1])) & 15) == 0 && (p.bDst & 1) == 0;
+        if (inten) grid.y = 1;                  // a pair holds both components
+        LineFn f = line_fn(p.N, d.axis != 0, inten ? 2 : (d.f1 && d.f2) ? 1 : 0, d.has_extra ? 2 : d.ang ? 1 : 0);
+        if (f == nullptr) return cudaErrorInvalidValue;
+        return launch_one(f, grid, dim3(p.T * p.G), smem, st, pdl, p);
+    } else {
+        const size_t smem = (size_t)p.L * p.P * sizeof(float2);
+        if (d.out_int || p.N != 16384 || smem > SRWG_LINE_SMEM_MAX) return cudaErrorInvalidValue;
+        LineFn f = d.has_extra ? line2e_get_14(d.axis != 0, d.f1, d.f2) : line2_get_14(d.axis != 0, d.f1, d.f2);
         if (f == nullptr) return cudaErrorInvalidValue;
         f<<<grid, p.T * p.L, smem, st>>>(p);
-    } else {
-        line_kernel<<<grid, p.T * p.G, smem, st>>>(p);
     }
     return cudaGetLastError();
 }

@@ -1,8 +1,10 @@
 // Launch parameters of the sm_100a kernels (kernels.cu).
 #pragma once
 #include <cuda_runtime.h>
+#include <vector>
 #include "kdesc.h"
 #include "linen_lengths.h"
+#include "linep_lengths.h"
 
 namespace srwg {
 
@@ -36,26 +38,36 @@ inline int line2_lines_per_cta(int axis, int N)
     return L;
 }
 
-struct LineLaunch {
-    LineDesc d;
+// what a line pass kernel takes (its descriptor stays in device memory)
+struct LineArgs {
     const float2* src[2];
     float2* dst[2];
-    const float2* tw;        // exp(-2 pi i k / N), k < N (FP64-accurate, rounded to FP32)
+    const float2* tw;        // the length's twiddle tables (line_twiddles)
     int N, nlines;           // line length, number of lines
-    int T, L, P, G;          // threads per line, lines per CTA, shared-memory pitch (float2), thread groups
-    int nst;
+    int T, L, P, G;          // threads per line (pair), lines per CTA, shared memory of one (float2; pairs:
+                             //   float4), lines (pairs) per CTA
+    int nst;                 // stages, their radices and (pairs, linep.cuh) lengths and reciprocals
     int radix[SRWG_MAX_STAGES];
-    int v2;                  // 1: power-of-two pass (line2_kernel), 2: general length (lineg_kernel),
-                             // 3: specialised general length (linen_kernel)
+    int len[SRWG_MAX_STAGES + 1];
+    unsigned dL[SRWG_MAX_STAGES + 1], dR[SRWG_MAX_STAGES], dB[SRWG_MAX_STAGES];
+    int tw1[SRWG_MAX_STAGES], tw2[SRWG_MAX_STAGES];
+    int pitch;               // pairs: pitch of the first digit's blocks
+    int alignIn, alignOut;   // pairs: 16-byte aligned fields (two lines at once)
+    int v2;                  // 0: pairs of lines (linep_kernel), 1: one line (line2_kernel, 16384 points)
     const float2* tabs;      // the plan's separable point-wise tables
     const LineDesc* gd;      // this pass's descriptor in device memory
+    int byValue;             // pairs: one descriptor for the whole launch, in `run` (else gd's)
+    LineRun run;
     int nb;                  // wavefronts in the launch (grid z; 0 or 1: one)
     long long bDesc, bTab;   // per wavefront: descriptor stride (bytes), table stride (float2)
     long long bSrc, bDst;    // per wavefront: source / destination field stride (float2)
-    int bulk;                // specialised pass: each CTA's input tile arrives by bulk async copies
+    int bulk;                // points of staging per component behind the slots (0: no bulk copies)
     int* status;             // device counter of waits that gave up (NULL: not recorded)
     long long spin;          // iteration limit of the bulk-copy wait
     int blk0, nblk;          // the line blocks launched: blk0 .. blk0 + nblk - 1 (nblk 0: all)
+};
+struct LineLaunch : LineArgs {
+    LineDesc d;              // host copy (launch shapes)
 };
 
 // tiled resize: a CTA makes TZ x TX new points from an old tile of at most OR_MAX x OC_MAX points
@@ -110,25 +122,24 @@ cudaError_t launch_moments(const MomLaunch& p, cudaStream_t st);
 cudaError_t launch_extract(const MomDesc& d, const MomDesc* gd, const float2* s0, const float2* s1,
                            const float2* tabs, char* out, cudaStream_t st);
 
-cudaError_t launch_line(const LineLaunch& p, cudaStream_t st);
+// pdl: the kernel may start while the one before it in the stream (a line pass or resize of the same run)
+// ends; it waits for it before it touches a field
+cudaError_t launch_line(const LineLaunch& p, cudaStream_t st, bool pdl = false);
+void fill_line_run(LineDesc& d);      // d.run from the rest of d (planner.cpp)
 
-// power-of-two line pass kernels, one translation unit per line length (line2_<logn>.cu)
-typedef void (*Line2Fn)(const LineLaunch);
-Line2Fn line2_kernel_ptr(int logn, bool cols, bool extra, int f1, int f2);
-#define SRWG_LINE2_DECL(L) Line2Fn line2_get_##L(bool cols, int f1, int f2); Line2Fn line2e_get_##L(bool cols, int f1, int f2);
-SRWG_LINE2_DECL(6) SRWG_LINE2_DECL(7) SRWG_LINE2_DECL(8) SRWG_LINE2_DECL(9) SRWG_LINE2_DECL(10)
-SRWG_LINE2_DECL(11) SRWG_LINE2_DECL(12) SRWG_LINE2_DECL(13) SRWG_LINE2_DECL(14)
-// general-length line pass kernels (lineg.cu, lineg_e.cu)
-Line2Fn lineg_get(bool cols);
-Line2Fn lineg_e_get(bool cols);
-// specialised general-length kernels (linen.cu, one unit per length of linen_lengths.h)
-#define SRWG_LINEN_DECL(N) Line2Fn linen_get_##N(bool cols, bool extra, int nt, bool inten);
-SRWG_LINEN_LENGTHS(SRWG_LINEN_DECL)
-SRWG_LINEN_POW2(SRWG_LINEN_DECL)
-#undef SRWG_LINEN_DECL
-Line2Fn linen_kernel_ptr(int N, bool cols, bool extra, int nt, bool inten = false);
+// line pass kernels: pairs of lines (linep.cu, one unit per axis and mode), 16384 points (line2_14.cu)
+typedef void (*LineFn)(const LineArgs);
+#define SRWG_LINEP_DECL(C, M) LineFn linep_get_##C##_##M(int extra);
+SRWG_LINEP_DECL(0, 0) SRWG_LINEP_DECL(0, 1) SRWG_LINEP_DECL(0, 2)
+SRWG_LINEP_DECL(1, 0) SRWG_LINEP_DECL(1, 1) SRWG_LINEP_DECL(1, 2)
+#undef SRWG_LINEP_DECL
+#define SRWG_LINEF_DECL(N, A, B, C, D, T) LineFn linef_get_##N(bool cols, int mode, int extra);
+SRWG_LINEF_LENGTHS(SRWG_LINEF_DECL)
+#undef SRWG_LINEF_DECL
+LineFn line2_get_14(bool cols, int f1, int f2);
+LineFn line2e_get_14(bool cols, int f1, int f2);
 inline bool line2_supported(int N) { return N >= 64 && N <= 16384 && (N & (N - 1)) == 0; }
-// general lengths of the specialised kernel
+// general lengths with launch shapes of their own in the tuning table
 inline bool linen_supported(int N)
 {
 #define SRWG_LINEN_IS(M) if (N == M) return true;
@@ -136,7 +147,6 @@ inline bool linen_supported(int N)
 #undef SRWG_LINEN_IS
     return false;
 }
-// powers of two that the specialised kernel is compiled for as well (the tuner's alternative)
 inline bool linen_pow2(int N)
 {
 #define SRWG_LINEN_IS(M) if (N == M) return true;
@@ -144,18 +154,15 @@ inline bool linen_pow2(int N)
 #undef SRWG_LINEN_IS
     return false;
 }
-// floats per thread that an intensity pass of the specialised kernel keeps between its two
-// components: the last stage's butterflies per thread times its radix (the radix schedule of
-// linen.cuh: radix-16 stages, one 8/4/2 stage, then 3, 5, 7; ceil(N/16) threads per line)
-__host__ __device__ constexpr int linen_int_floats(int N)
-{
-    int m = N, p2 = 0;
-    while (m % 2 == 0) { m /= 2; p2++; }
-    const int R = m % 7 == 0 ? 7 : m % 5 == 0 ? 5 : m % 3 == 0 ? 3 : (p2 % 4 ? 1 << (p2 % 4) : 16);
-    const int T = (N + 15) / 16;
-    return ((N / R + T - 1) / T) * R;
-}
-// line-pass kernel families (LineLaunch::v2)
+// lengths of the passes on pairs of lines: every even 2^a 3^b 5^c 7^d 11^e 13^f (e, f <= 1) from 4 to
+// 8192 (they take zero windows and column blocks, and write intensities)
+bool pair_supported(int N);
+// the twiddle tables of a line pass of N points, as its kernel reads them
+void line_twiddles(int N, std::vector<float2>& h);
+// columns that a column pass of N points transforms per CTA on a grid of nl columns: the width of
+// the column blocks the row pass before it writes (0: the pass is not one on pairs, or nl has no such blocks)
+int pair_block(int N, int nl);
+// kernel families of the tuning entry points
 enum { FAM_TAB = 0, FAM_POW2 = 1, FAM_GEN = 2, FAM_SPEC = 3 };
 // lines per CTA of the specialised general-length pass (at most 512 threads, 128 registers each):
 // rows up to 512 threads, columns a power of two up to 512 threads / 32 columns (the column-block
@@ -184,10 +191,8 @@ inline bool fixed_lines_valid(int axis, int N, int L, int fam)
     if (fam == FAM_SPEC && (linen_supported(N) || linen_pow2(N))) return ((N + 15) / 16) * L <= 512;
     return false;
 }
-// kernel family and lines per CTA of the line kernels with compile-time lengths (line2 / linen; they
-// skip a zero window and read / write column blocks): the autotuned choice where the tuning table has
-// one (capi.cpp), else the power-of-two kernel for powers of two and the specialised one for the
-// listed general lengths with the defaults above; lines 0 for other lengths
+// family and lines per CTA of the tuned lengths: the tuning table's choice where it has one
+// (capi.cpp), else the defaults above; lines 0 for other lengths
 int fixed_family(int axis, int N);
 int fixed_lines_per_cta(int axis, int N);
 cudaError_t launch_resize(const ResizeLaunch& p, cudaStream_t st);

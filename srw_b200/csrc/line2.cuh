@@ -130,7 +130,7 @@ __device__ __forceinline__ void fftN(float2* s, const float2* __restrict__ gin, 
 // quartic part of the angular transfer function); a separate instantiation keeps its registers out
 // of the common kernels
 template <int LOGN, bool COLS, bool EXTRA, int D1, int D2>
-__global__ void __launch_bounds__(1024, 1) line2_kernel(const LineLaunch p)
+__global__ void __launch_bounds__(1024, 1) line2_kernel(const LineArgs p)
 {
     constexpr int N = 1 << LOGN;
     constexpr int T = N / 16;
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(1024, 1) line2_kernel(const LineLaunch p)
 
 // kernel of a (COLS, EXTRA, f1, f2) combination
 template <int LOGN, bool COLS, bool EXTRA>
-Line2Fn line2_select(int f1, int f2)
+LineFn line2_select(int f1, int f2)
 {
     if (f1 > 0 && f2 > 0) return line2_kernel<LOGN, COLS, EXTRA, 1, 1>;
     if (f1 > 0 && f2 < 0) return line2_kernel<LOGN, COLS, EXTRA, 1, -1>;

@@ -3,7 +3,7 @@
 #include "line2.cuh"
 
 namespace srwg {
-Line2Fn line2_get_14(bool cols, int f1, int f2)
+LineFn line2_get_14(bool cols, int f1, int f2)
 {
     return cols ? line2_select<14, true, false>(f1, f2) : line2_select<14, false, false>(f1, f2);
 }

@@ -3,7 +3,7 @@
 #include "line2.cuh"
 
 namespace srwg {
-Line2Fn line2e_get_14(bool cols, int f1, int f2)
+LineFn line2e_get_14(bool cols, int f1, int f2)
 {
     return cols ? line2_select<14, true, true>(f1, f2) : line2_select<14, false, true>(f1, f2);
 }

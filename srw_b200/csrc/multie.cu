@@ -150,12 +150,11 @@ static void mark_intensity_pass(std::vector<KernelDesc>& ks, const std::vector<f
         LineDesc& d = ks[i].line;
         if (ks[i].kind == K_LINE && !d.has_extra && !(d.f1 && d.f2)) {
             const int N = d.axis == 0 ? d.nx : d.nz, nl = d.axis == 0 ? d.nz : d.nx;
-            if (fixed_family(d.axis, N) == FAM_SPEC) {
+            if (pair_supported(N)) {
                 d.out_int = 1;
                 // a column pass writes the intensity in blocks of its tile's columns (contiguous
                 // pieces); the accumulation reads that layout
-                const int bw = fixed_lines_per_cta(1, N);
-                if (d.axis == 1 && d.blk_out == 0 && bw > 1 && d.nx % bw == 0) d.blk_out = bw;
+                if (d.axis == 1 && d.blk_out == 0) d.blk_out = pair_block(N, d.nx);
                 const ChainTab& out = d.f1 ? d.t_mid : d.t_fin;
                 const double a = flat_mag2(tables, out.tab, N), b = flat_mag2(tables, d.t_pre.ltab, nl),
                              c = flat_mag2(tables, d.t_mid.ltab, nl), e = flat_mag2(tables, d.t_fin.ltab, nl);
@@ -163,6 +162,7 @@ static void mark_intensity_pass(std::vector<KernelDesc>& ks, const std::vector<f
                     d.int_flat = 1;
                     d.int_scale = (float)(a * b * c * e);
                 }
+                fill_line_run(d);
             }
         }
         return;
@@ -297,7 +297,7 @@ static bool same_structure(const std::vector<KernelDesc>& a, const std::vector<K
             const LineDesc &p = x.line, &q = y.line;
             if (p.axis != q.axis || p.nx != q.nx || p.nz != q.nz || p.f1 != q.f1 || p.f2 != q.f2 ||
                 p.has_extra != q.has_extra || p.zwin != q.zwin || p.blk_in != q.blk_in || p.blk_out != q.blk_out ||
-                p.out_int != q.out_int || p.int_flat != q.int_flat)
+                p.out_int != q.out_int || p.int_flat != q.int_flat || p.ang != q.ang)
                 return false;
         } else if (x.kind == K_RESIZE) {
             const ResizeDesc &p = x.rs, &q = y.rs;
@@ -502,7 +502,8 @@ extern "C" SRWG_API int srwgMultiECreate(const SRWLWfr* pBase, const SRWLOptC* p
     if (r) { set_last_detail(pl.err); delete m; return r; }
     m->nIn = (size_t)m->nx * m->nz;
     m->nOut = (size_t)pl.w.nx * pl.w.nz;
-    m->perWork = (size_t)std::max<long long>(pl.maxElems, 1);
+    m->perWork = (size_t)std::max<long long>(pl.maxElems, 2);
+    m->perWork += m->perWork & 1;        // 16-byte aligned fields
     const size_t tabBytes = ((pl.tables.size() * sizeof(float2) + 255) & ~(size_t)255) + 4096;   // slack for alignment pads
     m->descOff = tabBytes;
     m->constStride = (tabBytes + pl.kernels.size() * sizeof(KernelDesc) + 255) & ~(size_t)255;

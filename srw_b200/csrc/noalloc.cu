@@ -132,10 +132,9 @@ extern "C" SRWG_API int srwgPropagElecFieldStatic(const SRWLWfr* pWfr, const SRW
         if (twOff.count(N)) continue;
         while ((cst.size() * sizeof(float2)) % 256) cst.push_back(float2{0.f, 0.f});
         twOff[N] = cst.size();
-        for (int i = 0; i < N; i++) {
-            double a = -2. * M_PI * (double)i / (double)N;
-            cst.push_back(float2{(float)cos(a), (float)sin(a)});
-        }
+        std::vector<float2> tw;
+        line_twiddles(N, tw);
+        cst.insert(cst.end(), tw.begin(), tw.end());
     }
     if (cst.size() > SRWG_STATIC_CONST_POINTS) {
         set_last_detail("the plan's tables need " + std::to_string(cst.size()) + " points, above the static limit of " +
@@ -206,6 +205,8 @@ extern "C" SRWG_API int srwgPropagElecFieldStatic(const SRWLWfr* pWfr, const SRW
             p.src[0] = s0; p.src[1] = s1; p.dst[0] = d0; p.dst[1] = d1;
             p.tabs = cdev;
             p.gd = &gk[i].line;
+            p.byValue = 1;
+            p.run = k.line.run;
             e = launch_line(p, st);
         } else if (k.kind == K_RESIZE) {
             ResizeLaunch p;

@@ -150,13 +150,16 @@ static long long push(std::vector<float2>& T, const std::vector<cd>& v)
 
 // table of one chain W[k] = tab[k] * ltab[line] * extra * V[src(k)]:
 // [post of a previous transform: rs1 / shift1 / scale1] -> [pw] -> [mirror] -> [pre of the next: rs2 / shift2]
+// lin, alt: a further linear phase lin k and sign (-1)^k on the destination index
 static ChainTab chain_table(std::vector<float2>& T, int N, int nLine, int rs1, int sh1, double a1, float sc1,
-                            const SepPart* A, const SepPart* Lp, cd scale, int mir, int rs2, int sh2, double a2)
+                            const SepPart* A, const SepPart* Lp, cd scale, int mir, int rs2, int sh2, double a2,
+                            double lin = 0., int alt = 0)
 {
     ChainTab ct;
     ct.tab = -1;
     ct.ltab = -1;
-    bool along = rs1 || sh1 || sc1 != 1.f || (A && A->any) || rs2 || sh2 || scale != cd(1., 0.);
+    bool along = rs1 || sh1 || sc1 != 1.f || (A && A->any) || rs2 || sh2 || scale != cd(1., 0.) ||
+                 lin != 0. || alt;
     if (along) {
         std::vector<cd> v(N);
         std::vector<double> ph(N), sg(N);
@@ -167,6 +170,8 @@ static ChainTab chain_table(std::vector<float2>& T, int N, int nLine, int rs1, i
             int m = k;
             if (rs2) { m = k + half; if (m >= N) m -= N; if (k & 1) g = -g; }
             if (sh2) p += a2 * (double)(m - half);
+            p += lin * (double)k;
+            if (alt && (k & 1)) g = -g;
             int i = mir ? (N - 1 - m) : m;
             z[k] = 0;
             if (A) { p += A->ph[i]; z[k] = A->zero[i]; }
@@ -194,6 +199,48 @@ static ChainTab chain_table(std::vector<float2>& T, int N, int nLine, int rs1, i
         ct.ltab = push(T, v);
     }
     return ct;
+}
+
+// The quartic part of the angular transfer function (phase c0 q2 (c1 q2)(1 + 2 c1 q2), q2 = qx^2 + qz^2) as
+// the only non-separable work of a pass with two transforms: FP32 tables of qx^2 and qz^2 (from FP64)
+// along the line and per line instead of the point-by-point evaluation.  Where it is below 2^-27 rad
+// everywhere (a quarter of an FP32 rounding of the factor) it is dropped.
+static void quartic_tables(std::vector<float2>& T, LineDesc& d, int N, int nl)
+{
+    PwOps& e = d.extra;
+    if (!e.has_ang || e.has_bpx || e.has_tr || e.nmask) return;
+    const bool rows = d.axis == 0;
+    const double a0 = rows ? e.qx0 : e.qz0, da = rows ? e.dqx : e.dqz, l0 = rows ? e.qz0 : e.qx0, dl = rows ? e.dqz : e.dqx;
+    auto put = [&](int n, double q0, double dq, bool along, double& most) {
+        const size_t off = T.size();
+        T.resize(off + (n + 1) / 2);
+        float* f = reinterpret_cast<float*>(&T[off]);
+        for (int k = 0; k < n; k++) {
+            int i = k;
+            if (along) {                          // destination k of the middle chain is evaluated at mirror(rot(k))
+                if (d.f2_pre.rs) { i = k + N / 2; if (i >= N) i -= N; }
+                if (d.mirror_along) i = N - 1 - i;
+            }
+            const double q = q0 + (double)i * dq;
+            most = std::max(most, q * q);
+            f[k] = (float)(q * q);
+        }
+        return (int)off;
+    };
+    const size_t before = T.size();
+    double ma = 0., ml = 0.;
+    d.qtab = put(N, a0, da, true, ma);
+    d.qline = put(nl, l0, dl, false, ml);
+    d.qc0 = (float)e.c0;
+    d.qc1 = (float)e.c1;
+    const double q2 = ma + ml, c1q2 = std::fabs(e.c1 * q2), ph = std::fabs(e.c0 * q2) * c1q2 * (1. + 2. * c1q2);
+    d.has_extra = 0;
+    if (ph < 0x1p-27) {
+        T.resize(before);
+        d.ang = 0;
+    } else {
+        d.ang = ph < 0.03 ? 1 : 2;
+    }
 }
 
 // RadResizeCore (sroptelm.cpp:3038-3337) index arithmetic along one axis, in the reference's FP64
@@ -267,7 +314,7 @@ void build_tables(std::vector<KernelDesc>& ks, std::vector<float2>& T)
     // room for the largest tables the passes can ask for (no reallocation while they are added)
     size_t most = 0;
     for (const KernelDesc& k : ks) {
-        if (k.kind == K_LINE) most += 3 * (size_t)(k.line.nx + k.line.nz);
+        if (k.kind == K_LINE) most += 4 * (size_t)(k.line.nx + k.line.nz);
         else if (k.kind == K_RESIZE) most += 4 * (size_t)(k.rs.nxn + k.rs.nzn) + 2 * (size_t)(k.rs.nxo + k.rs.nzo) + 2;
         else if (reads_only(k.kind)) most += (size_t)(k.mom.nx + k.mom.nz);
         else most += (size_t)(k.pwk.nx + k.pwk.nz);
@@ -284,14 +331,31 @@ void build_tables(std::vector<KernelDesc>& ks, std::vector<float2>& T)
             if (d.has_pw) separate(d.pw, d.axis, N, nl, A, Lp, scale, d.extra, d.has_extra);
             const SepPart* pA = d.has_pw ? &A : nullptr;
             const SepPart* pL = d.has_pw ? &Lp : nullptr;
+            // Two transforms run through their middle chain in registers, output k to input k.  Where the
+            // chain's source is another index -- N - 1 - k (a mirror), k + N/2 (one centring rotation
+            // only) -- the first transform X is replaced by one that gives X[source(k)] at k:
+            // X[N - 1 - k] is the transform in the other direction of x[n] exp(2 pi i f1 n / N), and
+            // N/2 further is a factor (-1)^n on the input
+            d.dir1 = d.f1;
+            double lin = 0.;
+            int alt = 0;
+            if (d.f1 && d.f2 && pair_supported(N)) {
+                alt = (d.f1_post.rs != 0) != (d.f2_pre.rs != 0);
+                if (d.mirror_along) {
+                    d.dir1 = -d.f1;
+                    lin = 2. * M_PI * d.f1 / N;
+                }
+            }
             d.t_pre = chain_table(T, N, nl, 0, 0, 0., 1.f, nullptr, nullptr, cd(1., 0.), 0, d.f1_pre.rs,
-                                  d.f1_pre.has_shift, d.f1_pre.shift_a);
+                                  d.f1_pre.has_shift, d.f1_pre.shift_a, lin, alt);
             int rs1 = 0, sh1 = 0, rs2 = 0, sh2 = 0;
             double a1 = 0., a2 = 0.;
             float sc1 = 1.f;
             if (d.f1) { rs1 = d.f1_post.rs; sh1 = d.f1_post.has_shift; a1 = d.f1_post.shift_a; sc1 = d.f1_post.scale; }
             if (d.f2) { rs2 = d.f2_pre.rs; sh2 = d.f2_pre.has_shift; a2 = d.f2_pre.shift_a; }
             d.t_mid = chain_table(T, N, nl, rs1, sh1, a1, sc1, pA, pL, scale, d.mirror_along, rs2, sh2, a2);
+            d.ang = 0;
+            if (d.has_extra && d.f1 && d.f2 && pair_supported(N)) quartic_tables(T, d, N, nl);
             d.t_fin.tab = d.t_fin.ltab = -1;
             if (d.f2)
                 d.t_fin = chain_table(T, N, nl, d.f2_post.rs, d.f2_post.has_shift, d.f2_post.shift_a, d.f2_post.scale,
