@@ -261,22 +261,31 @@ SRWG_API int srwgMultiEDestroy(srwgMultiE* m);
  * factors pp[5..8] by hand): kernels of a small FP32 MLP and of the wavefront features it reads.
  * All pointers are device memory of the current device; row-major matrices.
  *   srwgMlpGemm:        C = alpha op(A) op(B) + beta C, op(A) M x K, op(B) K x N (trans flags transpose)
+ *   srwgMlpLinear:      Z = X W + bias, Y = act(Z) (X M x K, W K x N): a layer in one launch
+ *   srwgMlpLinearBackward: dW = X^T dZ and db = column sums of dZ in one launch and, with dX, dX = dZ W^T, times
+ *                       GELU'(Zprev) (M x K) when Zprev is given
  *   srwgMlpBiasAct:     Z += bias (per column); Y = act(Z), act 0 identity, 1 GELU (tanh form)
  *   srwgMlpActBackward: dY *= act'(Z)
  *   srwgMlpColSum:      db[j] = sum_i dZ[i][j]
  *   srwgMlpMse:         *loss += mean (out - target)^2 (FP64), dout = 2 (out - target) / n
- *   srwgMlpAdam:        Adam step t (>= 1) with bias correction
+ *   srwgMlpAdam:        Adam step t (>= 1) with bias correction; srwgMlpAdamMany: of n arrays, len[i] values each
  *   srwgWfrFeatures:    total intensity averaged on 64 x 64 cells (dFeat[4096]) and the sums of the
  *                       weighted fit of the phase curvature left after removing k (x^2/R0x + z^2/R0z)/2
  *                       (dSums[4]: sum w x dphi, sum w x^2, the same in z; k = 2 pi / lambda) */
 SRWG_API int srwgMlpGemm(int M, int N, int K, const float* A, int lda, int transA, const float* B, int ldb, int transB,
                          float* C, int ldc, float alpha, float beta, void* stream);
+SRWG_API int srwgMlpLinear(int M, int N, int K, const float* X, const float* W, const float* bias, float* Z, float* Y, int act,
+                           void* stream);
+SRWG_API int srwgMlpLinearBackward(int M, int N, int K, const float* X, const float* W, const float* dZ, float* dW, float* db,
+                                   float* dX, const float* Zprev, void* stream);
 SRWG_API int srwgMlpBiasAct(float* Z, const float* bias, float* Y, int M, int N, int act, void* stream);
 SRWG_API int srwgMlpActBackward(const float* Z, float* dY, long long n, int act, void* stream);
 SRWG_API int srwgMlpColSum(const float* dZ, float* db, int M, int N, void* stream);
 SRWG_API int srwgMlpMse(const float* out, const float* target, float* dout, double* loss, int n, void* stream);
 SRWG_API int srwgMlpAdam(float* w, const float* g, float* m, float* v, long long n, float lr, float b1, float b2,
                          float eps, int t, void* stream);
+SRWG_API int srwgMlpAdamMany(int n, float* const* w, const float* const* g, float* const* m, float* const* v,
+                             const long long* len, float lr, float b1, float b2, float eps, int t, void* stream);
 SRWG_API int srwgWfrFeatures(const float* dEx, const float* dEy, int nx, int ny, double xStart, double xStep,
                              double zStart, double zStep, double k, double invRx0, double invRz0, float* dFeat,
                              double* dSums, void* stream);

@@ -5,6 +5,7 @@
 // training loop and the memory they run on are driven from the host (srw_b200/learned.py).
 // Nothing here has a counterpart in the reference: it chooses the resize factors that the
 // reference's users set by hand in the propagation parameters (pp[5..8]).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -14,63 +15,9 @@
 #include "errors.h"
 #include "exec.h"
 
-namespace srwg {
+namespace cg = cooperative_groups;
 
-// C[M x N] = alpha * op(A) * op(B) + beta * C; op(A) is M x K (A row-major, lda; transposed when
-// transA), op(B) is K x N.  64 x 64 tile per CTA, K in steps of 16, 256 threads x 4 x 4 outputs.
-#define GT 64
-#define GK 16
-__global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, const float* __restrict__ A, int lda, int transA,
-                                                   const float* __restrict__ B, int ldb, int transB, float* __restrict__ C,
-                                                   int ldc, float alpha, float beta)
-{
-    __shared__ float As[GK][GT + 4];
-    __shared__ float Bs[GK][GT + 4];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int m0 = blockIdx.y * GT, n0 = blockIdx.x * GT;
-    float acc[4][4] = {{0.f}};
-    for (int k0 = 0; k0 < K; k0 += GK) {
-        // 64 x 16 tile of op(A) and 16 x 64 tile of op(B): 1024 elements each, 4 per thread
-        for (int e = threadIdx.x; e < GT * GK; e += 256) {
-            const int mm = e / GK, kk = e % GK;                 // A tile element (m0 + mm, k0 + kk)
-            const int gm = m0 + mm, gk = k0 + kk;
-            float a = 0.f;
-            if (gm < M && gk < K) a = transA ? A[(size_t)gk * lda + gm] : A[(size_t)gm * lda + gk];
-            As[kk][mm] = a;
-            const int kb = e / GT, nb = e % GT;                 // B tile element (k0 + kb, n0 + nb)
-            const int gkb = k0 + kb, gn = n0 + nb;
-            float b = 0.f;
-            if (gkb < K && gn < N) b = transB ? B[(size_t)gn * ldb + gkb] : B[(size_t)gkb * ldb + gn];
-            Bs[kb][nb] = b;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < GK; kk++) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int gm = m0 + ty * 4 + i;
-        if (gm >= M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int gn = n0 + tx * 4 + j;
-            if (gn >= N) continue;
-            float* c = &C[(size_t)gm * ldc + gn];
-            *c = alpha * acc[i][j] + (beta != 0.f ? beta * *c : 0.f);
-        }
-    }
-}
+namespace srwg {
 
 __device__ __forceinline__ float gelu(float z)
 {   // tanh form of GELU (Hendrycks & Gimpel 2016)
@@ -83,6 +30,120 @@ __device__ __forceinline__ float gelu_grad(float z)
     const float u = c * (z + 0.044715f * z * z * z);
     const float t = tanhf(u);
     return 0.5f * (1.f + t) + 0.5f * z * (1.f - t * t) * c * (1.f + 3.f * 0.044715f * z * z);
+}
+
+// What follows a product in its kernel: Z = alpha op(A) op(B) + beta C + bias (row broadcast) to C; with
+// act, Y = GELU(Z) beside it (act 0: Y = Z); with zgrad, Z *= GELU'(zgrad) (same layout as C); with
+// bsum, the column sums of op(B) (the bias gradients that go with a weight gradient)
+struct GemmTail {
+    const float* bias;
+    float* Y;
+    int act;
+    const float* zgrad;
+    float* bsum;
+};
+
+// op(A) is M x K (A row-major, lda; transposed when TA), op(B) is K x N.  A CTA makes a 32 x 64 tile over
+// one of gridDim.z pieces of K (steps of 32, the next step's operands loaded while this one is
+// multiplied); the pieces are the CTAs of a cluster, which then add their tiles through distributed
+// shared memory in piece order (no workspace, no atomics: the sum does not depend on scheduling).
+// The network's products are small and long: 128 x 256 with K = 4109 is 8 tiles of 64 x 64, whose 257
+// serial steps took 385 us; 16 tiles in 8 pieces occupy 128 SMs with 17 steps each.
+#define GM 32
+#define GN 64
+#define GK 32
+template <bool TA, bool TB>
+__global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, int kc, const float* __restrict__ A, int lda,
+                                                   const float* __restrict__ B, int ldb, float* __restrict__ C, int ldc,
+                                                   float alpha, float beta, const GemmTail t)
+{
+    __shared__ float As[2][GK][GM + 1];
+    __shared__ __align__(16) float Bs[2][GK][GN + 4];
+    __shared__ float cs[GN];
+    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+    const int m0 = blockIdx.x * GM, n0 = blockIdx.y * GN;
+    const int ka = blockIdx.z * kc, kb = min(K, ka + kc), nt = ka < kb ? (kb - ka + GK - 1) / GK : 0;
+    const bool sums = t.bsum != nullptr && blockIdx.x == 0;
+    float acc[2][4] = {{0.f}}, bs = 0.f;
+    float ra[4], rb[8];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int e = tid + 256 * i;
+            const int kk = TA ? e / GM : e % GK, mm = TA ? e % GM : e / GK;
+            const int gm = m0 + mm, gk = k0 + kk;
+            ra[i] = (gm < M && gk < kb) ? __ldg(&A[TA ? (size_t)gk * lda + gm : (size_t)gm * lda + gk]) : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int e = tid + 256 * i;
+            const int kk = TB ? e % GK : e / GN, nn = TB ? e / GK : e % GN;
+            const int gn = n0 + nn, gk = k0 + kk;
+            rb[i] = (gn < N && gk < kb) ? __ldg(&B[TB ? (size_t)gn * ldb + gk : (size_t)gk * ldb + gn]) : 0.f;
+        }
+    };
+    auto put = [&](int u) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int e = tid + 256 * i;
+            As[u][TA ? e / GM : e % GK][TA ? e % GM : e / GK] = ra[i];
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int e = tid + 256 * i;
+            Bs[u][TB ? e % GK : e / GN][TB ? e / GK : e % GN] = rb[i];
+        }
+    };
+    if (nt > 0) {
+        load(ka);
+        put(0);
+    }
+    __syncthreads();
+    for (int s = 0; s < nt; s++) {
+        const int u = s & 1;
+        if (s + 1 < nt) load(ka + (s + 1) * GK);
+#pragma unroll
+        for (int kk = 0; kk < GK; kk++) {
+            const float a0 = As[u][kk][ty * 2], a1 = As[u][kk][ty * 2 + 1];
+            const float4 b = *reinterpret_cast<const float4*>(&Bs[u][kk][tx * 4]);
+            acc[0][0] = fmaf(a0, b.x, acc[0][0]); acc[0][1] = fmaf(a0, b.y, acc[0][1]);
+            acc[0][2] = fmaf(a0, b.z, acc[0][2]); acc[0][3] = fmaf(a0, b.w, acc[0][3]);
+            acc[1][0] = fmaf(a1, b.x, acc[1][0]); acc[1][1] = fmaf(a1, b.y, acc[1][1]);
+            acc[1][2] = fmaf(a1, b.z, acc[1][2]); acc[1][3] = fmaf(a1, b.w, acc[1][3]);
+        }
+        if (sums && tid < GN)
+            for (int kk = 0; kk < GK; kk++) bs += Bs[u][kk][tid];
+        if (s + 1 < nt) put(u ^ 1);
+        __syncthreads();
+    }
+    // the piece's tile in shared memory (the operands are done with), then the sum over the cluster
+    float* red = &Bs[0][0][0];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) red[(ty * 2 + i) * GN + tx * 4 + j] = acc[i][j];
+    if (sums && tid < GN) cs[tid] = bs;
+    cg::cluster_group cl = cg::this_cluster();
+    cl.sync();
+    const int S = (int)cl.num_blocks(), r = (int)cl.block_rank();
+    for (int e = r * 256 + tid; e < GM * GN; e += S * 256) {
+        float v = 0.f;
+        for (int q = 0; q < S; q++) v += *cl.map_shared_rank(red + e, q);
+        const int gm = m0 + e / GN, gn = n0 + e % GN;
+        if (gm >= M || gn >= N) continue;
+        const size_t o = (size_t)gm * ldc + gn;
+        float z = alpha * v + (beta != 0.f ? beta * C[o] : 0.f);
+        if (t.bias) z += __ldg(&t.bias[gn]);
+        if (t.zgrad) z *= gelu_grad(__ldg(&t.zgrad[o]));
+        C[o] = z;
+        if (t.Y) t.Y[o] = t.act ? gelu(z) : z;
+    }
+    if (sums && r == 0 && tid < GN && n0 + tid < N) {
+        float v = 0.f;
+        for (int q = 0; q < S; q++) v += *cl.map_shared_rank(cs + tid, q);
+        t.bsum[n0 + tid] = v;
+    }
+    cl.sync();                    // no CTA leaves while another reads its tile
 }
 
 // Z[M x N] += bias (row broadcast); Y = act(Z) with act 0 = identity, 1 = GELU
@@ -104,14 +165,20 @@ __global__ void act_backward_kernel(const float* __restrict__ Z, float* __restri
     dY[i] *= gelu_grad(Z[i]);
 }
 
-// db[N] = sum over rows of dZ[M x N]
-__global__ void colsum_kernel(const float* __restrict__ dZ, float* __restrict__ db, int M, int N)
+// db[N] = sum over rows of dZ[M x N]: 32 columns per CTA, 8 partial sums each, added in order
+__global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ dZ, float* __restrict__ db, int M, int N)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= N) return;
+    __shared__ float part[8][33];
+    const int c = threadIdx.x & 31, g = threadIdx.x >> 5, j = blockIdx.x * 32 + c;
     float s = 0.f;
-    for (int i = 0; i < M; i++) s += dZ[(size_t)i * N + j];
-    db[j] = s;
+    if (j < N)
+        for (int i = g; i < M; i += 8) s += dZ[(size_t)i * N + j];
+    part[g][c] = s;
+    __syncthreads();
+    if (g == 0 && j < N) {
+        for (int k = 1; k < 8; k++) s += part[k][c];
+        db[j] = s;
+    }
 }
 
 // mean squared error over M x N: loss (one value, summed in FP64 per block then atomically) and
@@ -148,6 +215,32 @@ __global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, 
     m[i] = mi;
     v[i] = vi;
     w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+}
+
+// the same for several parameter arrays in one launch (element i of array k at index off[k] + i)
+#define ADAM_MOST 16
+struct AdamArrays {
+    float* w[ADAM_MOST];
+    const float* g[ADAM_MOST];
+    float* m[ADAM_MOST];
+    float* v[ADAM_MOST];
+    long long off[ADAM_MOST + 1];
+    int n;
+};
+__global__ void __launch_bounds__(256) adam_many_kernel(const AdamArrays a, float lr, float b1, float b2, float eps,
+                                                        float c1, float c2)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= a.off[a.n]) return;
+    int k = 0;
+    while (i >= a.off[k + 1]) k++;
+    const long long j = i - a.off[k];
+    const float gi = a.g[k][j];
+    const float mi = b1 * a.m[k][j] + (1.f - b1) * gi;
+    const float vi = b2 * a.v[k][j] + (1.f - b2) * gi * gi;
+    a.m[k][j] = mi;
+    a.v[k][j] = vi;
+    a.w[k][j] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
 }
 
 // features of one wavefront: total intensity averaged over 64 x 64 cells of the mesh (cell (cy, cx)
@@ -234,13 +327,70 @@ static int launch_status(cudaError_t e)
     return SRWG_ERR_CUDA;
 }
 
+static int gemm(int M, int N, int K, const float* A, int lda, int transA, const float* B, int ldb, int transB, float* C,
+                int ldc, float alpha, float beta, const GemmTail& t, cudaStream_t st)
+{
+    const int most = 65535 * GN;                 // columns of one launch
+    if (N > most) {
+        auto at = [](auto* q, int n) { return q ? q + n : q; };
+        for (int n = 0; n < N; n += most) {
+            const GemmTail u{at(t.bias, n), at(t.Y, n), t.act, at(t.zgrad, n), at(t.bsum, n)};
+            const int r = gemm(M, N - n < most ? N - n : most, K, A, lda, transA, transB ? B + (size_t)n * ldb : B + n, ldb,
+                               transB, C + n, ldc, alpha, beta, u, st);
+            if (r) return r;
+        }
+        return 0;
+    }
+    const int tm = (M + GM - 1) / GM, tn = (N + GN - 1) / GN;
+    // pieces of K: as many CTAs as two per SM, at least 64 steps of K each
+    int S = 8;
+    while (S > 1 && ((long long)tm * tn * S > 2 * 148 || K / S < 64)) S /= 2;
+    const int kc = (((K + S - 1) / S + GK - 1) / GK) * GK;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tm, tn, S);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = S;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaError_t e;
+    if (transA) {
+        if (transB) e = cudaLaunchKernelEx(&cfg, gemm_kernel<true, true>, M, N, K, kc, A, lda, B, ldb, C, ldc, alpha, beta, t);
+        else e = cudaLaunchKernelEx(&cfg, gemm_kernel<true, false>, M, N, K, kc, A, lda, B, ldb, C, ldc, alpha, beta, t);
+    } else {
+        if (transB) e = cudaLaunchKernelEx(&cfg, gemm_kernel<false, true>, M, N, K, kc, A, lda, B, ldb, C, ldc, alpha, beta, t);
+        else e = cudaLaunchKernelEx(&cfg, gemm_kernel<false, false>, M, N, K, kc, A, lda, B, ldb, C, ldc, alpha, beta, t);
+    }
+    return launch_status(e);
+}
+
 extern "C" SRWG_API int srwgMlpGemm(int M, int N, int K, const float* A, int lda, int transA, const float* B, int ldb,
                                     int transB, float* C, int ldc, float alpha, float beta, void* stream)
 {
     if (M <= 0 || N <= 0 || K <= 0 || !A || !B || !C) return SRWG_ERR_BAD_ARG;
-    dim3 grid((N + GT - 1) / GT, (M + GT - 1) / GT);
-    gemm_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(M, N, K, A, lda, transA, B, ldb, transB, C, ldc, alpha, beta);
-    return launch_status(cudaGetLastError());
+    return gemm(M, N, K, A, lda, transA, B, ldb, transB, C, ldc, alpha, beta, GemmTail{nullptr, nullptr, 0, nullptr, nullptr},
+                (cudaStream_t)stream);
+}
+
+extern "C" SRWG_API int srwgMlpLinear(int M, int N, int K, const float* X, const float* W, const float* bias, float* Z,
+                                      float* Y, int act, void* stream)
+{
+    if (M <= 0 || N <= 0 || K <= 0 || !X || !W || !bias || !Z || !Y) return SRWG_ERR_BAD_ARG;
+    return gemm(M, N, K, X, K, 0, W, N, 0, Z, N, 1.f, 0.f, GemmTail{bias, Y, act, nullptr, nullptr}, (cudaStream_t)stream);
+}
+
+extern "C" SRWG_API int srwgMlpLinearBackward(int M, int N, int K, const float* X, const float* W, const float* dZ,
+                                              float* dW, float* db, float* dX, const float* Zprev, void* stream)
+{
+    if (M <= 0 || N <= 0 || K <= 0 || !X || !dZ || !dW || !db || (dX && !W)) return SRWG_ERR_BAD_ARG;
+    int r = gemm(K, N, M, X, K, 1, dZ, N, 0, dW, N, 1.f, 0.f, GemmTail{nullptr, nullptr, 0, nullptr, db}, (cudaStream_t)stream);
+    if (r == 0 && dX)
+        r = gemm(M, K, N, dZ, N, 0, W, N, 1, dX, K, 1.f, 0.f, GemmTail{nullptr, nullptr, 0, Zprev, nullptr},
+                 (cudaStream_t)stream);
+    return r;
 }
 
 extern "C" SRWG_API int srwgMlpBiasAct(float* Z, const float* bias, float* Y, int M, int N, int act, void* stream)
@@ -261,7 +411,7 @@ extern "C" SRWG_API int srwgMlpActBackward(const float* Z, float* dY, long long 
 extern "C" SRWG_API int srwgMlpColSum(const float* dZ, float* db, int M, int N, void* stream)
 {
     if (M <= 0 || N <= 0 || !dZ || !db) return SRWG_ERR_BAD_ARG;
-    colsum_kernel<<<(N + 255) / 256, 256, 0, (cudaStream_t)stream>>>(dZ, db, M, N);
+    colsum_kernel<<<(N + 31) / 32, 256, 0, (cudaStream_t)stream>>>(dZ, db, M, N);
     return launch_status(cudaGetLastError());
 }
 
@@ -279,6 +429,26 @@ extern "C" SRWG_API int srwgMlpAdam(float* w, const float* g, float* m, float* v
     const float c1 = 1.f - powf(b1, (float)t), c2 = 1.f - powf(b2, (float)t);
     adam_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(w, g, m, v, (size_t)n, lr, b1, b2, eps, c1,
                                                                               c2);
+    return launch_status(cudaGetLastError());
+}
+
+extern "C" SRWG_API int srwgMlpAdamMany(int n, float* const* w, const float* const* g, float* const* m, float* const* v,
+                                        const long long* len, float lr, float b1, float b2, float eps, int t, void* stream)
+{
+    if (n <= 0 || !w || !g || !m || !v || !len || t < 1) return SRWG_ERR_BAD_ARG;
+    for (int i = 0; i < n; i++)
+        if (len[i] <= 0 || !w[i] || !g[i] || !m[i] || !v[i]) return SRWG_ERR_BAD_ARG;
+    const float c1 = 1.f - powf(b1, (float)t), c2 = 1.f - powf(b2, (float)t);
+    for (int i0 = 0; i0 < n; i0 += ADAM_MOST) {
+        AdamArrays a;
+        a.n = n - i0 < ADAM_MOST ? n - i0 : ADAM_MOST;
+        a.off[0] = 0;
+        for (int i = 0; i < a.n; i++) {
+            a.w[i] = w[i0 + i]; a.g[i] = g[i0 + i]; a.m[i] = m[i0 + i]; a.v[i] = v[i0 + i];
+            a.off[i + 1] = a.off[i] + len[i0 + i];
+        }
+        adam_many_kernel<<<(unsigned)((a.off[a.n] + 255) / 256), 256, 0, (cudaStream_t)stream>>>(a, lr, b1, b2, eps, c1, c2);
+    }
     return launch_status(cudaGetLastError());
 }
 

@@ -94,11 +94,10 @@ class ResizeMLP(object):
         for l, (W, b) in enumerate(zip(self.W, self.b)):
             B, n_out = a.shape[0], W.shape[1]
             z = self.torch.empty((B, n_out), dtype=self.torch.float32, device=self.dev)
-            _check(L.srwgMlpGemm(B, n_out, a.shape[1], a.data_ptr(), a.shape[1], 0, W.data_ptr(), n_out, 0,
-                                 z.data_ptr(), n_out, 1.0, 0.0, st), 'mlp gemm')
             y = self.torch.empty_like(z)
             act = 1 if l + 1 < len(self.W) else 0
-            _check(L.srwgMlpBiasAct(z.data_ptr(), b.data_ptr(), y.data_ptr(), B, n_out, act, st), 'mlp bias')
+            _check(L.srwgMlpLinear(B, n_out, a.shape[1], a.data_ptr(), W.data_ptr(), b.data_ptr(), z.data_ptr(),
+                                   y.data_ptr(), act, st), 'mlp layer')
             self.Z.append(z)
             self.Y.append(y)
             a = y
@@ -112,23 +111,17 @@ class ResizeMLP(object):
         db = [None] * len(self.W)
         d = dOut.contiguous()
         for l in range(len(self.W) - 1, -1, -1):
-            act = 1 if l + 1 < len(self.W) else 0
-            if act:
-                _check(L.srwgMlpActBackward(self.Z[l].data_ptr(), d.data_ptr(), d.numel(), act, st), 'mlp act')
             a = self.Y[l]
             B, n_in, n_out = a.shape[0], a.shape[1], d.shape[1]
             gw = self.torch.empty((n_in, n_out), dtype=self.torch.float32, device=self.dev)
-            _check(L.srwgMlpGemm(n_in, n_out, B, a.data_ptr(), n_in, 1, d.data_ptr(), n_out, 0, gw.data_ptr(),
-                                 n_out, 1.0, 0.0, st), 'mlp dW')
             gb = self.torch.empty(n_out, dtype=self.torch.float32, device=self.dev)
-            _check(L.srwgMlpColSum(d.data_ptr(), gb.data_ptr(), B, n_out, st), 'mlp db')
+            # the gradient with respect to this layer's input, through the activation below it
+            da = self.torch.empty((B, n_in), dtype=self.torch.float32, device=self.dev) if l > 0 else None
+            _check(L.srwgMlpLinearBackward(B, n_out, n_in, a.data_ptr(), self.W[l].data_ptr(), d.data_ptr(),
+                                           gw.data_ptr(), gb.data_ptr(), da.data_ptr() if l > 0 else None,
+                                           self.Z[l - 1].data_ptr() if l > 0 else None, st), 'mlp layer gradients')
             dW[l], db[l] = gw, gb
-            if l > 0:
-                da = self.torch.empty((B, n_in), dtype=self.torch.float32, device=self.dev)
-                W = self.W[l]
-                _check(L.srwgMlpGemm(B, n_in, n_out, d.data_ptr(), n_out, 0, W.data_ptr(), n_out, 1, da.data_ptr(),
-                                     n_in, 1.0, 0.0, st), 'mlp dA')
-                d = da
+            d = da
         return dW, db
 
     def loss_grad(self, out, target):
@@ -145,9 +138,11 @@ class ResizeMLP(object):
         L = capi.lib()
         st = self._st()
         self.t += 1
-        for p, g, m, v in zip(self.W + self.b, dW + db, self.mW + self.mb, self.vW + self.vb):
-            _check(L.srwgMlpAdam(p.data_ptr(), g.data_ptr(), m.data_ptr(), v.data_ptr(), p.numel(), lr, b1, b2, eps,
-                                 self.t, st), 'mlp adam')
+        ps, gs, ms, vs = self.W + self.b, dW + db, self.mW + self.mb, self.vW + self.vb
+        n = len(ps)
+        arr = lambda ts: (C.c_void_p * n)(*[t.data_ptr() for t in ts])  # noqa: E731
+        _check(L.srwgMlpAdamMany(n, arr(ps), arr(gs), arr(ms), arr(vs), (C.c_longlong * n)(*[p.numel() for p in ps]), lr,
+                                 b1, b2, eps, self.t, st), 'mlp adam')
 
     def set_normalisation(self, X):
         self.xmean = X.mean(0)
