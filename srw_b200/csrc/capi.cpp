@@ -304,41 +304,31 @@ static int upload_tables(const Planner& pl, float2** buf, size_t* capElems, cuda
     return 0;
 }
 
-// runs a pass list on nb wavefronts at once: buffer 0 = input (wavefront b at inX + b * inStride), 1/2 =
-// work buffers (layout [buffer][component][wavefront][workElems]); the last pass writes the output
-// (outX + b * outStride).  dconst holds per wavefront (stride constStride bytes) the tables and, at
-// descOff, the pass descriptors; all wavefronts have passes of the same kinds and sizes.
-// a row pass whose lines outside its window are zero and read by nothing (zskip) launches only the
-// window's line blocks; `d` holds the window of the launch (for a batch: the union of its electrons')
+// a pass whose lines outside its window are zero and read by nothing (zskip) launches only the window's
+// line blocks; `d` holds the widest window of the launch (its wavefronts' windows start where each
+// one's descriptor says, so that a batch of shifted ones launches no blocks outside them)
 void line_window(const LineDesc& d, LineLaunch& p)
 {
-    if (d.zwin && d.zskip && d.zl0 <= d.zl1 && p.L > 0) {
-        const int l0 = std::max(0, d.zl0), l1 = std::min(p.nlines - 1, d.zl1);
-        if (l0 <= l1) {
-            p.blk0 = l0 / p.L;
-            p.nblk = l1 / p.L - p.blk0 + 1;
-        }
-    }
+    if (d.zwin && d.zskip && d.zl0 <= d.zl1 && p.L > 0) p.nblk = (d.zl1 - d.zl0 + p.L - 1) / p.L + 1;
 }
 
 // a tiled resize that writes only its window launches only the window's tiles
 void resize_window(const ResizeDesc& r, ResizeLaunch& p)
 {
-    if (!r.skip_zero || r.tile_or <= 0) return;
-    const long xs = std::max(0L, r.ixStart), xe = std::min((long)r.nxn - 1, r.ixEnd);
-    const long zs = std::max(0L, r.izStart), ze = std::min((long)r.nzn - 1, r.izEnd);
-    if (xs > xe || zs > ze) return;
-    p.tx0 = (int)(xs / SRWG_RESIZE_TX);
-    p.ntx = (int)(xe / SRWG_RESIZE_TX) - p.tx0 + 1;
-    p.tz0 = (int)(zs / SRWG_RESIZE_TZ);
-    p.ntz = (int)(ze / SRWG_RESIZE_TZ) - p.tz0 + 1;
+    if (!r.skip_zero || r.tile_or <= 0 || r.ixStart > r.ixEnd || r.izStart > r.izEnd) return;
+    p.ntx = (int)((r.ixEnd - r.ixStart + SRWG_RESIZE_TX - 1) / SRWG_RESIZE_TX) + 1;
+    p.ntz = (int)((r.izEnd - r.izStart + SRWG_RESIZE_TZ - 1) / SRWG_RESIZE_TZ) + 1;
 }
 
+// runs a pass list on nb wavefronts at once: buffer 0 = input (wavefront b at inX + b * inStride), 1/2 =
+// work buffers (layout [buffer][component][wavefront][workElems]); the last pass writes the output
+// (outX + b * outStride).  dconst holds per wavefront (stride constStride bytes) the tables and, at
+// descOff, the pass descriptors; all wavefronts have passes of the same kinds and sizes.
 int execute_passes(const std::vector<KernelDesc>& ks, DeviceCtx& c, int nb, const float2* inX, const float2* inY,
                    long long inStride, float2* outX, float2* outY, long long outStride, float2* work, size_t workElems,
                    const char* dconst, long long constStride, size_t descOff, cudaStream_t st, cudaEvent_t* ev,
                    const std::vector<KernelDesc>* hostMax, double* momScratch, double* momSlots, int nSlots,
-                   char* intOut)
+                   char* intOut, size_t nRun)
 {
     const size_t nk = ks.size();
     const size_t W = (size_t)nb * workElems;
@@ -351,7 +341,7 @@ int execute_passes(const std::vector<KernelDesc>& ks, DeviceCtx& c, int nb, cons
     for (size_t i = nk; i-- > 0;)
         if (!reads_only(ks[i].kind)) { lastField = i; break; }
 
-    for (size_t i = 0; i < nk; i++) {
+    for (size_t i = 0; i < nk && i < nRun; i++) {
         const KernelDesc& k = hostMax ? (*hostMax)[i] : ks[i];
         if (ev) CUDA_TRY(cudaEventRecord(ev[2 * i], st));
         const bool fromOut = reads_only(k.kind) && k.src != 0 && i > lastField && k.src == ks[lastField].dst;

@@ -84,13 +84,15 @@ struct alignas(16) LineRun {
     int mirror_lines;
     int zwin, zl0, zl1, za0, za1, zskip;
     int blk_in, blk_out;
+    int in_p, in_l0, in_q0;         // storage of the input: pitch, first stored line, first stored point
+    int out_p, out_l0;              // of the output: pitch, first stored line (see LineDesc)
     int extra;                      // the middle chain has non-separable work
     int int_flat;
     float int_scale;
     int ang;                        // quartic part of the angular transfer function in the middle chain (two
     int qtab, qline;                //   transforms): 0 none, 1 |phase| < 0.03, 2 any; tables of q^2 (floats)
     float qc0, qc1;                 //   along the line and per line, phase = qc0 q2 (qc1 q2)(1 + 2 qc1 q2)
-    int pad[2];
+    int pad[1];
 };
 
 struct LineDesc {
@@ -118,7 +120,14 @@ struct LineDesc {
                                     //   column intensity pass (out_int): the intensity of column c at
                                     //   point i at ((c / blk_out) N + i) blk_out + c % blk_out
     int blk_in;                     // column pass: input in blocks of blk_in columns (0: row-major)
-    int out_int;                    // last pass of a multi-electron batch on a specialised kernel: one
+    // Windowed fields are stored without what is known to be zero.  Input: in_p points between rows
+    // (row-major) or between blocks (per column of a block), starting at line in_l0, point in_q0; output:
+    // the stored lines out_l0 .. out_l0 + out_p - 1 (columns: between rows; blocks: columns per block).
+    // in_p, out_p 0: the whole grid.
+    int in_p, in_l0, in_q0, out_p, out_l0;
+    int out_int;                    // (2: along the rows, only those the detector samples, fused with the
+                                    //   accumulation: linep_sample_kernel)
+                                    // last pass of a multi-electron batch on pairs: one
                                     //   CTA transforms both components of its lines and writes the
                                     //   total intensity |Ex|^2 + |Ey|^2 (float, dst[0]) instead of them
     int ang, qtab, qline;           // see LineRun
@@ -149,6 +158,7 @@ struct ResizeDesc {
                                                //   tile of new points (0: not tiled)
     int skip_zero;                             // points outside the window are not written: the next
                                                //   pass treats them as zero (LineDesc::zwin)
+    int cp, cx0, cz0;                          // storage of the new points: pitch, first column and row
 };
 
 // per new-mesh index along one axis: first old node of the 4-point stencil, clipped relative cell

@@ -312,7 +312,9 @@ __global__ void __launch_bounds__(256) resize2_kernel(const ResizeLaunch p)
     float2* old = reinterpret_cast<float2*>(H + 2 * OR * TX);   // [comp][old row][old column]
     __shared__ int ext[4];
     const int tid = threadIdx.x;
-    const int x0 = (blockIdx.x + p.tx0) * TX, z0 = (blockIdx.y + p.tz0) * TZ;
+    // a resize that writes only its window starts at this wavefront's first tile of it
+    const int x0 = (blockIdx.x + (d.skip_zero ? max(0, (int)d.ixStart) / TX : 0)) * TX;
+    const int z0 = (blockIdx.y + (d.skip_zero ? max(0, (int)d.izStart) / TZ : 0)) * TZ;
     const int xa = max(x0, (int)d.ixStart), xb = min(min(x0 + TX, d.nxn) - 1, (int)d.ixEnd);
     const int za = max(z0, (int)d.izStart), zb = min(min(z0 + TZ, d.nzn) - 1, (int)d.izEnd);
     if (xa > xb || za > zb) {
@@ -447,7 +449,7 @@ __global__ void __launch_bounds__(256) resize2_kernel(const ResizeLaunch p)
                 out[1] = cmul(out[1], f);
             }
         }
-        const size_t o = (size_t)gj * d.nxn + gi;
+        const size_t o = d.cp ? (size_t)(gj - d.cz0) * d.cp + (gi - d.cx0) : (size_t)gj * d.nxn + gi;
         __stcs(&D[0][o], out[0]);
         __stcs(&D[1][o], out[1]);
     }
@@ -522,13 +524,7 @@ cudaError_t launch_line(const LineLaunch& pin, cudaStream_t st, bool pdl)
     LineArgs p = pin;
     const LineDesc& d = pin.d;
     dim3 grid((p.nlines + p.L - 1) / p.L, 2, p.nb > 1 ? p.nb : 1);
-    if (p.nblk > 0) {
-        // only the line blocks of the window (the others would write nothing)
-        if (p.blk0 < 0 || p.blk0 + p.nblk > (int)grid.x) return cudaErrorInvalidValue;
-        grid.x = p.nblk;
-    } else {
-        p.blk0 = 0;
-    }
+    if (p.nblk > 0) grid.x = std::min((int)grid.x, p.nblk);      // only the window's line blocks
     if (attrs_needed(0)) {
         const int dirs[8][2] = {{1, 1}, {1, -1}, {-1, 1}, {-1, -1}, {1, 0}, {-1, 0}, {0, 1}, {0, -1}};
         for (int e = 0; e < 2; e++) {
@@ -586,6 +582,50 @@ cudaError_t launch_line(const LineLaunch& pin, cudaStream_t st, bool pdl)
     return cudaGetLastError();
 }
 
+static SampleFn sample_fn(int N)
+{
+    switch (N) {
+#define SRWG_LINEF_CASE(M, A, B, C, D, T) case M: return lines_get_##M();
+    SRWG_LINEF_LENGTHS(SRWG_LINEF_CASE)
+#undef SRWG_LINEF_CASE
+    default: return lines_get();
+    }
+}
+
+// two pairs' slots, two intensity rows, the detector row's sums
+static size_t sample_smem(const LineLaunch& p, int anx)
+{
+    return (size_t)2 * p.P * sizeof(float4) + (size_t)(2 * p.N + (p.N & 1) * 2) * sizeof(float) + (size_t)anx * sizeof(double);
+}
+bool sample_fits(const LineLaunch& p, int anx)
+{
+    return p.v2 == 0 && 2 * p.T <= 512 && sample_smem(p, anx) <= SRWG_LINE_SMEM_MAX;
+}
+
+cudaError_t launch_line_sample(const LineLaunch& p, const SampleArgs& q, cudaStream_t st, bool pdl)
+{
+    if (!sample_fits(p, q.anx) || p.d.axis != 0 || p.d.has_extra || p.d.ang || (p.d.f1 && p.d.f2) || q.per < 1)
+        return cudaErrorInvalidValue;
+    if (attrs_needed(2)) {
+#define SRWG_LINEF_ATTR(M, A, B, C, D, T)                                                                   \
+        cudaFuncSetAttribute(lines_get_##M(), cudaFuncAttributeMaxDynamicSharedMemorySize, SRWG_LINE_SMEM_MAX);
+        SRWG_LINEF_LENGTHS(SRWG_LINEF_ATTR)
+#undef SRWG_LINEF_ATTR
+        cudaFuncSetAttribute(lines_get(), cudaFuncAttributeMaxDynamicSharedMemorySize, SRWG_LINE_SMEM_MAX);
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(q.anz, (q.nb + q.per - 1) / q.per);
+    cfg.blockDim = dim3(2 * p.T);
+    cfg.dynamicSmemBytes = sample_smem(p, q.anx);
+    cfg.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, sample_fn(p.N), (const LineArgs&)p, q);
+}
+
 cudaError_t launch_resize(const ResizeLaunch& q, cudaStream_t st)
 {
     ResizeLaunch p = q;
@@ -601,14 +641,9 @@ cudaError_t launch_resize(const ResizeLaunch& q, cudaStream_t st)
         dim3 grid((p.d.nxn + SRWG_RESIZE_TX - 1) / SRWG_RESIZE_TX, (p.d.nzn + SRWG_RESIZE_TZ - 1) / SRWG_RESIZE_TZ,
                   p.nb > 1 ? p.nb : 1);
         ResizeLaunch q = p;
-        if (p.ntx > 0 && p.ntz > 0) {
-            // only the tiles of the window (the others would write nothing)
-            if (p.tx0 < 0 || p.tz0 < 0 || p.tx0 + p.ntx > (int)grid.x || p.tz0 + p.ntz > (int)grid.y)
-                return cudaErrorInvalidValue;
-            grid.x = p.ntx;
-            grid.y = p.ntz;
-        } else {
-            q.tx0 = q.tz0 = 0;
+        if (p.ntx > 0 && p.ntz > 0) {            // only the window's tiles
+            grid.x = std::min((int)grid.x, p.ntx);
+            grid.y = std::min((int)grid.y, p.ntz);
         }
         resize2_kernel<<<grid, 256, smem, st>>>(q);
         return cudaGetLastError();

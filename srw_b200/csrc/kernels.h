@@ -64,10 +64,29 @@ struct LineArgs {
     int bulk;                // points of staging per component behind the slots (0: no bulk copies)
     int* status;             // device counter of waits that gave up (NULL: not recorded)
     long long spin;          // iteration limit of the bulk-copy wait
-    int blk0, nblk;          // the line blocks launched: blk0 .. blk0 + nblk - 1 (nblk 0: all)
+    int nblk;                // line blocks launched, from the window's first one (0: all)
 };
 struct LineLaunch : LineArgs {
     LineDesc d;              // host copy (launch shapes)
+};
+
+// per-electron parameters of a multi-electron batch in device memory
+struct ElecParams {
+    double kx, kz;                       // kick: phase kx x + kz z on the base mesh (fused by the planner)
+    double dx, dz;                       // mesh shift of the electron's wavefront
+    double oxStart, oxStep, ozStart, ozStep;   // output mesh (steps as (Fin - Start)/(n - 1))
+    double oxInv, ozInv;                       // 1 / step: the accumulation multiplies (no FP64 divisions)
+    int onx, onz;
+    int pad[2];
+};
+
+// the sampled last pass of a multi-electron batch (linep_sample_kernel): detector mesh, electrons per
+// CTA, and the groups' sums [groups][anz][anx]
+struct SampleArgs {
+    const ElecParams* ep;
+    double* part;
+    int nb, per, anx, anz;
+    double axStart, axStep, azStart, azStep;
 };
 
 // tiled resize: a CTA makes TZ x TX new points from an old tile of at most OR_MAX x OC_MAX points
@@ -87,7 +106,7 @@ struct ResizeLaunch {
     int nb;                  // wavefronts in the launch (grid z; 0 or 1: one)
     long long bDesc, bTab;   // per wavefront: descriptor stride (bytes), table stride (float2)
     long long bSrc, bDst;    // per wavefront: source / destination field stride (float2)
-    int tx0, tz0, ntx, ntz;  // tiled kernel: the tiles launched (first, count per axis; ntx 0: all)
+    int ntx, ntz;            // tiled kernel: tiles launched per axis, from the window's first ones (0: all)
 };
 
 struct PwLaunch {
@@ -125,15 +144,20 @@ cudaError_t launch_extract(const MomDesc& d, const MomDesc* gd, const float2* s0
 // pdl: the kernel may start while the one before it in the stream (a line pass or resize of the same run)
 // ends; it waits for it before it touches a field
 cudaError_t launch_line(const LineLaunch& p, cudaStream_t st, bool pdl = false);
+// the sampled row pass of a batch; its shape (threads, shared memory) must fit: sample_fits
+cudaError_t launch_line_sample(const LineLaunch& p, const SampleArgs& q, cudaStream_t st, bool pdl);
+bool sample_fits(const LineLaunch& p, int anx);
 void fill_line_run(LineDesc& d);      // d.run from the rest of d (planner.cpp)
 
 // line pass kernels: pairs of lines (linep.cu, one unit per axis and mode), 16384 points (line2_14.cu)
 typedef void (*LineFn)(const LineArgs);
+typedef void (*SampleFn)(const LineArgs, const SampleArgs);
+SampleFn lines_get();
 #define SRWG_LINEP_DECL(C, M) LineFn linep_get_##C##_##M(int extra);
 SRWG_LINEP_DECL(0, 0) SRWG_LINEP_DECL(0, 1) SRWG_LINEP_DECL(0, 2)
 SRWG_LINEP_DECL(1, 0) SRWG_LINEP_DECL(1, 1) SRWG_LINEP_DECL(1, 2)
 #undef SRWG_LINEP_DECL
-#define SRWG_LINEF_DECL(N, A, B, C, D, T) LineFn linef_get_##N(bool cols, int mode, int extra);
+#define SRWG_LINEF_DECL(N, A, B, C, D, T) LineFn linef_get_##N(bool cols, int mode, int extra); SampleFn lines_get_##N();
 SRWG_LINEF_LENGTHS(SRWG_LINEF_DECL)
 #undef SRWG_LINEF_DECL
 LineFn line2_get_14(bool cols, int f1, int f2);

@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(1024, 1) line2_kernel(const LineArgs p)
     const int tid = threadIdx.x;
     const int g = COLS ? (tid % L) : (tid / T);          // line of the tile
     const int t = COLS ? (tid / L) : (tid - g * T);      // thread within the line
-    const int bx = blockIdx.x + p.blk0;                 // line block
+    const int bx = blockIdx.x;                          // line block
     const int line = bx * L + g;
     bool active = line < nl;
     float2* s = sm + (size_t)g * P;

@@ -35,10 +35,14 @@ LineFn SRWG_CATF(linef_get_, SRWG_LINEF_N)(bool cols, int mode, int extra)
     static_assert(Z::N() == SRWG_LINEF_N, "schedule");
     return cols ? pick<Z, true>(mode, extra) : pick<Z, false>(mode, extra);
 }
+SampleFn SRWG_CATF(lines_get_, SRWG_LINEF_N)() { return linep_sample_kernel<FixedOf<SRWG_LINEF_N>::Z>; }
 #else
 LineFn SRWG_CAT(linep_get_, SRWG_LINEP_COLS, SRWG_LINEP)(int extra)
 {
     return pick_extra<PShape, SRWG_LINEP_COLS != 0, SRWG_LINEP>(extra);
 }
+#if SRWG_LINEP == 2 && SRWG_LINEP_COLS == 0
+SampleFn lines_get() { return linep_sample_kernel<PShape>; }
+#endif
 #endif
 }  // namespace srwg

@@ -96,6 +96,18 @@ __device__ __forceinline__ float4 ldfield4(const float2* p)
     asm volatile("ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
     return v;
 }
+// the same where `on`, else v stays (one predicated instruction: no branch, so that a butterfly's loads
+// are in flight together)
+__device__ __forceinline__ void ldfield_if(bool on, const float2* p, float& x, float& y)
+{
+    asm volatile("{ .reg .pred q; setp.ne.b32 q, %3, 0; @q ld.global.L1::no_allocate.v2.f32 {%0, %1}, [%2]; }"
+                 : "+f"(x), "+f"(y) : "l"(p), "r"((int)on));
+}
+__device__ __forceinline__ void ldfield4_if(bool on, const float2* p, float4& v)
+{
+    asm volatile("{ .reg .pred q; setp.ne.b32 q, %5, 0; @q ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4]; }"
+                 : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w) : "l"(p), "r"((int)on));
+}
 __device__ __forceinline__ float2 f2sub(float2 a, float2 b)
 {
     unsigned long long r;
@@ -399,6 +411,7 @@ struct PLine {
     const float2* tabs;
     const PwOps* ex;
     int line0, line1;
+    float* si;              // intensity line in shared memory
     bool has_lf;
     float2 lfr, lfi;        // line factors
     const float* qtab;      // quartic angular term (EXTRA 1): q^2 along the line, of the two lines, coefficients
@@ -502,24 +515,27 @@ __device__ __forceinline__ void pload(P2 (&v)[R], const PLine& x, const PChain& 
         const unsigned oA = x.ioff + (unsigned)((q0 + hs) * gs), oB = x.ioff + (unsigned)((q0 - hs) * gs);
         const unsigned os = (unsigned)(qs * gs);
         const int wA = q0 + hs - x.za0, wB = q0 - hs - x.za0;
+        auto in = [&](int r) { return (unsigned)((r < R / 2 ? wA : wB) + r * qs) <= x.zn; };
+        auto at = [&](int r) { return (r < R / 2 ? oA : oB) + (unsigned)r * os; };
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-            const bool in = (unsigned)((r < R / 2 ? wA : wB) + r * qs) <= x.zn;
-            const unsigned o = (r < R / 2 ? oA : oB) + (unsigned)r * os;
-            a[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (x.sg0 != nullptr) {
+        for (int r = 0; r < R; r++) a[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (x.sg0 != nullptr) {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
                 const int e = ((r < R / 2 ? wA : wB) + r * qs) * gs;
-                float2 t0 = make_float2(0.f, 0.f), t1 = t0;
-                if (in && x.in0) t0 = x.sg0[e];
-                if (in && x.in1) t1 = x.sg1[e];
-                a[r] = make_float4(t0.x, t0.y, t1.x, t1.y);
-            } else if (VEC && x.vin) {
-                if (in) a[r] = ldfield4(x.g0 + o);
-            } else {
-                float2 t0 = make_float2(0.f, 0.f), t1 = t0;
-                if (in && x.in0) t0 = ldfield(x.g0 + o);
-                if (in && x.in1) t1 = ldfield(x.g1 + o);
-                a[r] = make_float4(t0.x, t0.y, t1.x, t1.y);
+                if (in(r)) {
+                    const float2 t0 = x.sg0[e], t1 = x.sg1[e];
+                    a[r] = make_float4(t0.x, t0.y, t1.x, t1.y);
+                }
+            }
+        } else if (VEC && x.vin) {
+#pragma unroll
+            for (int r = 0; r < R; r++) ldfield4_if(in(r), x.g0 + at(r), a[r]);
+        } else {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                ldfield_if(in(r) && x.in0, x.g0 + at(r), a[r].x, a[r].y);
+                ldfield_if(in(r) && x.in1, x.g1 + at(r), a[r].z, a[r].w);
             }
         }
     }
@@ -528,7 +544,7 @@ __device__ __forceinline__ void pload(P2 (&v)[R], const PLine& x, const PChain& 
         v[r].re = make_float2(a[r].x, a[r].z);
         v[r].im = make_float2(a[r].y, a[r].w);
     }
-    if (VEC && x.vin && !(x.in0 && x.in1)) {        // a pair at the edge of the window: one line is zero
+    if (!(x.in0 && x.in1) && !x.full) {              // a pair at the edge of the window: one line is zero
 #pragma unroll
         for (int r = 0; r < R; r++) {
             v[r].re = make_float2(x.in0 ? v[r].re.x : 0.f, x.in1 ? v[r].re.y : 0.f);
@@ -547,15 +563,10 @@ __device__ __forceinline__ void pload(P2 (&v)[R], const PLine& x, const PChain& 
     if (cj < 0.f) pconj(v);
 }
 
-// one output of both lines: factors, then the stores at p0 and p1; OUTI: the intensity of the pair
-// (both components) as one float
-template <bool COLS, int EXTRA, bool OUTI>
-__device__ __forceinline__ void pput(P2 o, const PLine& x, const PChain& c, int kk, const float2* tb, void* p0, float2* p1,
-                                     int N, float iscale)
+// one output of both lines to p0 and p1; OUTI: the intensity of the pair (both components) as one float
+template <bool COLS, int OUTI>
+__device__ __forceinline__ void pput(const P2& o, const PLine& x, void* p0, float2* p1, float iscale)
 {
-    if (c.tab >= 0) o = pmul(o, __ldg(tb));
-    if (EXTRA == 2 && c.extra) o = pextra<COLS>(o, x, pindex(c, kk, N));
-    if (x.has_lf) o = pmul2(o, x.lfr, x.lfi);
     if (OUTI) {
         const float2 I = __ffma2_rn(o.im, o.im, __fmul2_rn(o.re, o.re));
         if (x.st0) __stcs(reinterpret_cast<float*>(p0), (I.x + I.y) * iscale);
@@ -567,12 +578,56 @@ __device__ __forceinline__ void pput(P2 o, const PLine& x, const PChain& c, int 
     }
 }
 
-// the R outputs u + r M of a line's last stage to global memory through the output chain
-template <int R, bool COLS, int EXTRA, bool OUTI>
+// the output chain's factors on the R outputs with destinations kk(r): the table's values are loaded
+// together (a load per output between its stores waited for each in turn)
+template <int R, bool COLS, int EXTRA, class KK>
+__device__ __forceinline__ void pfactors(P2 (&v)[R], const PLine& x, const PChain& c, int N, const KK& kk)
+{
+    if (c.tab >= 0) {
+        const float2* tb = x.tabs + c.tab;
+        constexpr int H = R > 8 ? (R + 1) / 2 : R;       // (more at once does not fit the registers)
+#pragma unroll
+        for (int r0 = 0; r0 < R; r0 += H) {
+            float2 f[H];
+#pragma unroll
+            for (int r = 0; r < H; r++)
+                if (r0 + r < R) f[r] = __ldg(tb + kk(r0 + r));
+#pragma unroll
+            for (int r = 0; r < H; r++)
+                if (r0 + r < R) v[r0 + r] = pmul(v[r0 + r], f[r]);
+        }
+    }
+    if (EXTRA == 2 && c.extra) {
+#pragma unroll
+        for (int r = 0; r < R; r++) v[r] = pextra<COLS>(v[r], x, pindex(c, kk(r), N));
+    }
+    if (x.has_lf) {
+#pragma unroll
+        for (int r = 0; r < R; r++) v[r] = pmul2(v[r], x.lfr, x.lfi);
+    }
+}
+
+// the R outputs u + r M of a line's last stage through the output chain: OUTI 0 the fields, 1 the intensity
+// of the pair (both components) to global memory, 2 that intensity to shared memory
+template <int R, bool COLS, int EXTRA, int OUTI>
 __device__ __forceinline__ void pstore(P2 (&v)[R], const PLine& x, const PChain& c, int u, int M, int N, float cj,
                                        float iscale)
 {
     if (cj < 0.f) pconj(v);
+    if constexpr (OUTI == 2) {
+        // the intensity of the pair, in shared memory
+        auto kk = [&](int r) {
+            const int k = prot(u + r * M, N, c.rot_out);
+            return c.mir ? N - 1 - k : k;
+        };
+        pfactors<R, COLS, EXTRA>(v, x, c, N, kk);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const float2 I = __ffma2_rn(v[r].im, v[r].im, __fmul2_rn(v[r].re, v[r].re));
+            x.si[kk(r)] = (I.x + I.y) * iscale;
+        }
+        return;
+    }
     constexpr int EB = OUTI ? 4 : 8;                     // bytes of an output element
     const int h = c.rot_out ? (N >> 1) : 0;
     char* b0 = reinterpret_cast<char*>(x.o0);
@@ -582,31 +637,32 @@ __device__ __forceinline__ void pstore(P2 (&v)[R], const PLine& x, const PChain&
         // (the upper half's base may lie before the field: signed distances)
         const long long eA = ((long long)x.ooff + (u + h)) * EB, eB = ((long long)x.ooff + (u - h)) * EB;
         char *pA = b0 + eA, *pB = b0 + eB, *qA = b1 + eA, *qB = b1 + eB;
-        const float2 *tA = x.tabs + c.tab + u + h, *tB = x.tabs + c.tab + u - h;
+        pfactors<R, COLS, EXTRA>(v, x, c, N, [&](int r) { return (r < R / 2 ? u + h : u - h) + r * M; });
 #pragma unroll
         for (int r = 0; r < R; r++)
-            pput<COLS, EXTRA, OUTI>(v[r], x, c, (r < R / 2 ? u + h : u - h) + r * M, (r < R / 2 ? tA : tB) + r * M,
-                                    (r < R / 2 ? pA : pB) + r * M * EB,
-                                    reinterpret_cast<float2*>((r < R / 2 ? qA : qB) + r * M * EB), N, iscale);
+            pput<COLS, OUTI>(v[r], x, (r < R / 2 ? pA : pB) + r * M * EB,
+                             reinterpret_cast<float2*>((r < R / 2 ? qA : qB) + r * M * EB), iscale);
     } else if ((R % 2 == 0 || h == 0) && (x.lg < 0 || (M & ((1 << x.lg) - 1)) == 0)) {
         // destinations and their places are a base (per half of r) plus r steps
         const int kA = c.mir ? N - 1 - (u + h) : u + h, kB = c.mir ? N - 1 - (u - h) : u - h, ks = c.mir ? -M : M;
         const unsigned pA = x.ooff + (unsigned)x.place(kA), pB = x.ooff + (unsigned)x.place(kB);
         const unsigned ps = (unsigned)(x.lg < 0 ? ks * x.ostr : (ks >> x.lg) * x.bstr);
+        pfactors<R, COLS, EXTRA>(v, x, c, N, [&](int r) { return (r < R / 2 ? kA : kB) + r * ks; });
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            const int kk = (r < R / 2 ? kA : kB) + r * ks;
             const unsigned o = (r < R / 2 ? pA : pB) + (unsigned)r * ps;
-            pput<COLS, EXTRA, OUTI>(v[r], x, c, kk, x.tabs + c.tab + kk, b0 + (size_t)o * EB,
-                                    reinterpret_cast<float2*>(b1 + (size_t)o * EB), N, iscale);
+            pput<COLS, OUTI>(v[r], x, b0 + (size_t)o * EB, reinterpret_cast<float2*>(b1 + (size_t)o * EB), iscale);
         }
     } else {
+        auto kk = [&](int r) {
+            const int k = prot(u + r * M, N, c.rot_out);
+            return c.mir ? N - 1 - k : k;
+        };
+        pfactors<R, COLS, EXTRA>(v, x, c, N, kk);
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            const int k = prot(u + r * M, N, c.rot_out), kk = c.mir ? N - 1 - k : k;
-            const unsigned o = x.ooff + (unsigned)x.place(kk);
-            pput<COLS, EXTRA, OUTI>(v[r], x, c, kk, x.tabs + c.tab + kk, b0 + (size_t)o * EB,
-                                    reinterpret_cast<float2*>(b1 + (size_t)o * EB), N, iscale);
+            const unsigned o = x.ooff + (unsigned)x.place(kk(r));
+            pput<COLS, OUTI>(v[r], x, b0 + (size_t)o * EB, reinterpret_cast<float2*>(b1 + (size_t)o * EB), iscale);
         }
     }
 }
@@ -663,7 +719,7 @@ __device__ __forceinline__ void run_mid(const Z& z, int st, float4* s, const flo
     }
 }
 
-template <int R, class Z, bool COLS, int EXTRA, bool OUTI>
+template <int R, class Z, bool COLS, int EXTRA, int OUTI>
 __device__ __forceinline__ void run_last(const Z& z, float4* s, const PLine& x, const PChain& c, float cj,
                                          float iscale, int t)
 {
@@ -764,7 +820,8 @@ __global__ void __launch_bounds__(512, 1) linep_kernel(const LineArgs p)
     const int N = z.N(), nl = p.nlines, Lp = p.G, tid = threadIdx.x;
     const int g = COLS ? tid % Lp : tid / z.T();
     const int t = COLS ? tid / Lp : tid - g * z.T();
-    const int bx = blockIdx.x + p.blk0;
+    // a pass that writes only its window's lines starts at this wavefront's first block of them
+    const int bx = blockIdx.x + (d.zwin && d.zskip ? d.zl0 / p.L : 0);
     PLine x;
     int line0 = (bx * Lp + g) * LPP;
     const bool valid = line0 < nl;
@@ -773,15 +830,16 @@ __global__ void __launch_bounds__(512, 1) linep_kernel(const LineArgs p)
     x.line1 = INT ? line0 : line0 + 1;                   // (pairs: an even number of lines)
     x.st0 = x.st1 = valid;
     float4* s = smp + g * p.P;
-    // input: row-major, or (column pass after a row pass) blocks of blk_in columns stored together
-    x.gstr = COLS ? nl : 1;
-    x.ioff = COLS ? (unsigned)line0 : (unsigned)line0 * (unsigned)N;
+    // input: row-major, or blocks of blk_in lines stored together; only the window where it is stored alone
+    const int ip = d.in_p;
+    x.gstr = COLS ? ip : 1;
+    x.ioff = COLS ? (unsigned)(line0 - d.in_l0 - d.in_q0 * ip) : (unsigned)((line0 - d.in_l0) * ip - d.in_q0);
     x.g0 = src;
-    x.g1 = src + (COLS || d.blk_in > 0 ? 1 : N);
+    x.g1 = src + (COLS || d.blk_in > 0 ? 1 : ip);
     bool pairIn = COLS || d.blk_in > 0;
     if (d.blk_in > 0) {
         x.gstr = d.blk_in;
-        x.ioff = (unsigned)(line0 / d.blk_in) * (unsigned)(N * d.blk_in) + (unsigned)(line0 % d.blk_in);
+        x.ioff = (unsigned)((line0 / d.blk_in * ip - d.in_q0) * d.blk_in + line0 % d.blk_in);
     }
     if (INT) {
         x.g1 = p.src[1] + blockIdx.z * p.bSrc;
@@ -789,17 +847,18 @@ __global__ void __launch_bounds__(512, 1) linep_kernel(const LineArgs p)
     }
     x.vin = pairIn && p.alignIn;
     const int o0 = d.mirror_lines ? nl - 1 - line0 : line0, od = d.mirror_lines ? -1 : 1;
-    x.ooff = COLS ? (unsigned)o0 : (unsigned)o0 * (unsigned)N;
-    x.ostr = COLS ? nl : 1;
+    const int op = d.out_p;
+    x.ooff = COLS ? (unsigned)(o0 - d.out_l0) : (unsigned)((o0 - d.out_l0) * op);
+    x.ostr = COLS ? op : 1;
     x.lg = -1;
     x.bstr = 0;
     x.o0 = dst;
-    x.o1 = dst + (COLS ? od : od * N);
+    x.o1 = dst + (COLS ? od : od * op);
     x.vout = COLS && p.alignOut && od == 1;
     if (!INT && d.blk_out > 0) {
         x.lg = 31 - __clz(d.blk_out);
-        x.bstr = nl * d.blk_out;
-        x.ooff = (unsigned)o0 * (unsigned)d.blk_out;
+        x.bstr = op * d.blk_out;
+        x.ooff = (unsigned)((o0 - d.out_l0) * d.blk_out);
         x.o1 = dst + od * d.blk_out;
         x.vout = 0;
     }
@@ -850,7 +909,7 @@ __global__ void __launch_bounds__(512, 1) linep_kernel(const LineArgs p)
         float2* stg = reinterpret_cast<float2*>(smp + Lp * p.P);
         const int pts = (d.za1 - d.za0 + 1) * p.L;
         if (pts <= p.bulk) {
-            const size_t o = (size_t)bx * N * p.L + (size_t)d.za0 * p.L;
+            const size_t o = ((size_t)bx * ip + (d.za0 - d.in_q0)) * p.L;
             if (tid == 0) {
                 mbar_init(&bar);
                 mbar_expect(&bar, (unsigned)(pts * sizeof(float2)) * (INT ? 2 : 1));
@@ -879,16 +938,6 @@ __global__ void __launch_bounds__(512, 1) linep_kernel(const LineArgs p)
         x.has_lf = false;
         iscale = d.int_scale;
     }
-    // line factors: loaded here, multiplied before the last stage
-    float2 fa[3], fb[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        fa[k] = fb[k] = make_float2(1.f, 0.f);
-        if (x.has_lf && d.lt[k] >= 0) {
-            fa[k] = __ldg(&x.tabs[d.lt[k] + line0]);
-            fb[k] = __ldg(&x.tabs[d.lt[k] + x.line1]);
-        }
-    }
     if (EXTRA == 1) {
         x.qtab = reinterpret_cast<const float*>(x.tabs + d.qtab);
         const float* ql = reinterpret_cast<const float*>(x.tabs + d.qline);
@@ -897,6 +946,18 @@ __global__ void __launch_bounds__(512, 1) linep_kernel(const LineArgs p)
         x.qc1 = d.qc1;
         x.qsmall = d.ang == 1;
     }
+    // line factors: loaded before the last barrier, multiplied after it
+    float2 fa[3], fb[3];
+    auto load_factors = [&]() {
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            fa[k] = fb[k] = make_float2(1.f, 0.f);
+            if (x.has_lf && d.lt[k] >= 0) {
+                fa[k] = __ldg(&x.tabs[d.lt[k] + line0]);
+                fb[k] = __ldg(&x.tabs[d.lt[k] + x.line1]);
+            }
+        }
+    };
     auto line_factors = [&]() {
         const float2 a = cmul(cmul(fa[0], fa[1]), fa[2]), b = cmul(cmul(fb[0], fb[1]), fb[2]);
         x.lfr = make_float2(a.x, b.x);
@@ -914,47 +975,175 @@ __global__ void __launch_bounds__(512, 1) linep_kernel(const LineArgs p)
     if constexpr (Z::fixed) {
         constexpr int n = Z::n(), RA = Z::R(0), RB = Z::R(1), RC = Z::R(2), RL = Z::R(Z::n() - 1);
         run_first<RA, Z, COLS, EXTRA, !INT>(z, s, x, cin, cjin, tw, t);
-        __syncthreads();
-        if constexpr (n >= 3) { run_mid<RB, Z, true>(z, 1, s, tw, t); __syncthreads(); }
-        if constexpr (n >= 4) { run_mid<RC, Z, true>(z, 2, s, tw, t); __syncthreads(); }
+        if constexpr (n >= 3) { __syncthreads(); run_mid<RB, Z, true>(z, 1, s, tw, t); }
+        if constexpr (n >= 4) { __syncthreads(); run_mid<RC, Z, true>(z, 2, s, tw, t); }
         if constexpr (MODE != 1) {
-            line_factors();
-            run_last<RL, Z, COLS, EXTRA, INT>(z, s, x, cout, cjin, iscale, t);
-        } else {
-            run_turn<RL, Z, COLS, EXTRA>(z, s, x, mid, c1, c2, tw, t);
+            load_factors();
             __syncthreads();
-            if constexpr (n >= 4) { run_mid<RC, Z, false>(z, 2, s, tw, t); __syncthreads(); }
-            if constexpr (n >= 3) { run_mid<RB, Z, false>(z, 1, s, tw, t); __syncthreads(); }
+            line_factors();
+            run_last<RL, Z, COLS, EXTRA, INT ? 1 : 0>(z, s, x, cout, cjin, iscale, t);
+        } else {
+            __syncthreads();
+            run_turn<RL, Z, COLS, EXTRA>(z, s, x, mid, c1, c2, tw, t);
+            if constexpr (n >= 4) { __syncthreads(); run_mid<RC, Z, false>(z, 2, s, tw, t); }
+            if constexpr (n >= 3) { __syncthreads(); run_mid<RB, Z, false>(z, 1, s, tw, t); }
+            load_factors();
+            __syncthreads();
             line_factors();
             run_back<RA, Z, COLS, EXTRA>(z, s, x, fin, c2, t);
         }
     } else {
 #define LINEP_FIRST(R_) case R_: run_first<R_, Z, COLS, EXTRA, !INT>(z, s, x, cin, cjin, tw, t); break;
         switch (z.R(0)) { LINEP_EVEN(LINEP_FIRST) default: break; }
-        __syncthreads();
         for (int st = 1; st + 1 < z.n(); st++) {
+            __syncthreads();
 #define LINEP_MID(R_) case R_: run_mid<R_, Z, true>(z, st, s, tw, t); break;
             switch (z.R(st)) { LINEP_ALL(LINEP_MID) default: break; }
-            __syncthreads();
         }
         if constexpr (MODE != 1) {
+            load_factors();
+            __syncthreads();
             line_factors();
-#define LINEP_LAST(R_) case R_: run_last<R_, Z, COLS, EXTRA, INT>(z, s, x, cout, cjin, iscale, t); break;
+#define LINEP_LAST(R_) case R_: run_last<R_, Z, COLS, EXTRA, INT ? 1 : 0>(z, s, x, cout, cjin, iscale, t); break;
             switch (z.R(z.n() - 1)) { LINEP_ALL(LINEP_LAST) default: break; }
         } else {
+            __syncthreads();
 #define LINEP_TURN(R_) case R_: run_turn<R_, Z, COLS, EXTRA>(z, s, x, mid, c1, c2, tw, t); break;
             switch (z.R(z.n() - 1)) { LINEP_ALL(LINEP_TURN) default: break; }
-            __syncthreads();
             for (int st = z.n() - 2; st >= 1; st--) {
+                __syncthreads();
 #define LINEP_MID2(R_) case R_: run_mid<R_, Z, false>(z, st, s, tw, t); break;
                 switch (z.R(st)) { LINEP_ALL(LINEP_MID2) default: break; }
-                __syncthreads();
             }
+            load_factors();
+            __syncthreads();
             line_factors();
 #define LINEP_BACK(R_) case R_: run_back<R_, Z, COLS, EXTRA>(z, s, x, fin, c2, t); break;
             switch (z.R(0)) { LINEP_EVEN(LINEP_BACK) default: break; }
         }
     }
+}
+
+// Last pass of a multi-electron batch along the rows, fused with the accumulation: only the rows the
+// detector samples are transformed.  A CTA makes one detector row for several electrons in turn: the
+// two output rows around it (one pair of both components per row), their intensities in shared
+// memory, bilinear interpolation onto the detector row (avg_update_interp, order 1: nothing outside an
+// electron's mesh) in FP64, summed over the CTA's electrons in their order; the groups' sums are added
+// by accum_parts_kernel.  At 1536 x 1600 on 512^2 (a detector row per 5 output rows) it transforms 640 of
+// the 1600 rows and writes no intensities.
+template <class Z>
+__global__ void __launch_bounds__(512, 1) linep_sample_kernel(const LineArgs p, const SampleArgs q)
+{
+    extern __shared__ float4 smp[];
+    Z z;
+    if constexpr (!Z::fixed) {
+        z.N_ = p.N; z.n_ = p.nst; z.T_ = p.T; z.pitch_ = p.pitch;
+        z.R_ = p.radix; z.L_ = p.len; z.dL = p.dL; z.dR = p.dR; z.dB = p.dB; z.t1 = p.tw1; z.t2 = p.tw2;
+    }
+    const int N = z.N(), nl = p.nlines, tid = threadIdx.x;
+    const int g = tid / z.T(), t = tid - g * z.T();      // g: the output row below / above the detector row
+    const int j = blockIdx.x, b1 = min(q.nb, (int)(blockIdx.y + 1) * q.per);
+    float4* s = smp + g * p.P;
+    float* I0 = reinterpret_cast<float*>(smp + 2 * p.P);
+    float* I1 = I0 + N;
+    double* acc = reinterpret_cast<double*>(I0 + 2 * N + (N & 1) * 2);
+    for (int i = tid; i < q.anx; i += blockDim.x) acc[i] = 0.;
+    const double y = q.azStart + (double)j * q.azStep;
+    PLine x;
+    x.g0 = x.g1 = nullptr;
+    x.sg0 = x.sg1 = nullptr;
+    x.o0 = x.o1 = nullptr;
+    x.ooff = 0;
+    x.ostr = 1; x.lg = -1; x.bstr = 0;
+    x.st0 = x.st1 = true;
+    x.vin = x.vout = 0;
+    x.ex = nullptr;
+    x.si = g ? I1 : I0;
+    const float2* tw = p.tw;
+    pdl_wait();
+    for (int b = blockIdx.y * q.per; b < b1; b++) {
+        const ElecParams& e = q.ep[b];
+        const int iy0 = (int)trunc((y - e.ozStart) * e.ozInv + 1.e-09);
+        if (iy0 < 0 || iy0 >= e.onz - 1) continue;
+        const LineRun d = reinterpret_cast<const LineDesc*>(reinterpret_cast<const char*>(p.gd) + b * p.bDesc)->run;
+        const int row = iy0 + g, line = d.mirror_lines ? nl - 1 - row : row;
+        x.line0 = x.line1 = line;
+        x.g0 = p.src[0] + b * p.bSrc;
+        x.g1 = p.src[1] + b * p.bSrc;
+        x.gstr = d.blk_in > 0 ? d.blk_in : 1;
+        x.ioff = d.blk_in > 0 ? (unsigned)((line / d.blk_in * d.in_p - d.in_q0) * d.blk_in + line % d.blk_in)
+                              : (unsigned)((line - d.in_l0) * d.in_p - d.in_q0);
+        x.za0 = 0;
+        x.zn = N - 1;
+        x.in0 = true;
+        x.full = d.blk_in == 0;
+        if (d.zwin) {
+            x.full = false;
+            x.in0 = line >= d.zl0 && line <= d.zl1 && d.za0 <= d.za1;
+            x.za0 = d.za0;
+            x.zn = (unsigned)max(d.za1 - d.za0, 0);
+        }
+        x.in1 = x.in0;
+        x.tabs = p.tabs + b * p.bTab;
+        PChain pre, mid, fin;
+        pre.rot_in = d.pre_rot; pre.mir = 0; pre.rot_out = 0; pre.tab = d.pre_tab; pre.extra = 0;
+        mid.rot_in = d.mid_in; mid.mir = d.mid_mir; mid.rot_out = d.mid_out; mid.tab = d.mid_tab; mid.extra = 0;
+        fin.rot_in = 0; fin.mir = 0; fin.rot_out = d.fin_rot; fin.tab = d.fin_tab; fin.extra = 0;
+        const bool one = d.dir1 != 0;
+        x.has_lf = d.lt[0] >= 0;
+        float iscale = 1.f;
+        if (d.int_flat) {
+            if (one) mid.tab = -1;
+            else fin.tab = -1;
+            x.has_lf = false;
+            iscale = d.int_scale;
+        }
+        x.lfr = make_float2(1.f, 1.f);
+        x.lfi = make_float2(0.f, 0.f);
+        if (x.has_lf) {
+            float2 a = make_float2(1.f, 0.f);
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+                if (d.lt[k] >= 0) a = cmul(a, __ldg(&x.tabs[d.lt[k] + line]));
+            x.lfr = make_float2(a.x, a.x);
+            x.lfi = make_float2(a.y, a.y);
+        }
+        const PChain cin = one ? pre : mid, cout = one ? mid : fin;
+        const float cj = (one ? d.dir1 : d.dir2) < 0 ? -1.f : 1.f;
+        if constexpr (Z::fixed) {
+            constexpr int n = Z::n(), RA = Z::R(0), RB = Z::R(1), RC = Z::R(2), RL = Z::R(Z::n() - 1);
+            run_first<RA, Z, false, 0, false>(z, s, x, cin, cj, tw, t);
+            if constexpr (n >= 3) { __syncthreads(); run_mid<RB, Z, true>(z, 1, s, tw, t); }
+            if constexpr (n >= 4) { __syncthreads(); run_mid<RC, Z, true>(z, 2, s, tw, t); }
+            __syncthreads();
+            run_last<RL, Z, false, 0, 2>(z, s, x, cout, cj, iscale, t);
+        } else {
+#define LINEP_SFIRST(R_) case R_: run_first<R_, Z, false, 0, false>(z, s, x, cin, cj, tw, t); break;
+            switch (z.R(0)) { LINEP_EVEN(LINEP_SFIRST) default: break; }
+            for (int st = 1; st + 1 < z.n(); st++) {
+                __syncthreads();
+#define LINEP_SMID(R_) case R_: run_mid<R_, Z, true>(z, st, s, tw, t); break;
+                switch (z.R(st)) { LINEP_ALL(LINEP_SMID) default: break; }
+            }
+            __syncthreads();
+#define LINEP_SLAST(R_) case R_: run_last<R_, Z, false, 0, 2>(z, s, x, cout, cj, iscale, t); break;
+            switch (z.R(z.n() - 1)) { LINEP_ALL(LINEP_SLAST) default: break; }
+        }
+        __syncthreads();
+        // (the next electron's first barrier comes before its intensities)
+        const double ty = (y - (e.ozStart + e.ozStep * iy0)) * e.ozInv;
+        for (int i = tid; i < q.anx; i += blockDim.x) {
+            const double xx = q.axStart + (double)i * q.axStep;
+            const int ix0 = (int)trunc((xx - e.oxStart) * e.oxInv + 1.e-09);
+            if (ix0 < 0 || ix0 >= e.onx - 1) continue;
+            const double tx = (xx - (e.oxStart + e.oxStep * ix0)) * e.oxInv;
+            const double a00 = I0[ix0], f10 = I0[ix0 + 1], f01 = I1[ix0], f11 = I1[ix0 + 1];
+            const double a10 = f10 - a00, a01 = f01 - a00, a11 = a00 - f01 - f10 + f11;
+            acc[i] += a00 + tx * (a10 + ty * a11) + ty * a01;
+        }
+    }
+    double* part = q.part + ((size_t)blockIdx.y * q.anz + j) * q.anx;
+    for (int i = tid; i < q.anx; i += blockDim.x) part[i] = acc[i];
 }
 
 }  // namespace srwg

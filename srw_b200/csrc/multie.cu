@@ -37,16 +37,6 @@
 
 namespace srwg {
 
-// per-electron parameters in device memory
-struct ElecParams {
-    double kx, kz;                       // kick: phase kx x + kz z on the base mesh (fused by the planner)
-    double dx, dz;                       // mesh shift of the electron's wavefront
-    double oxStart, oxStep, ozStart, ozStep;   // output mesh (steps as (Fin - Start)/(n - 1))
-    double oxInv, ozInv;                       // 1 / step: the accumulation multiplies (no FP64 divisions)
-    int onx, onz;
-    int pad[2];
-};
-
 // acc[p] += sum over the batch of the bilinearly interpolated total intensity at common-mesh
 // point p (avg_update_interp, order 1: points outside an electron's mesh add nothing)
 __global__ void __launch_bounds__(256) accum_kernel(const float2* __restrict__ ex, const float2* __restrict__ ey,
@@ -123,6 +113,17 @@ __global__ void __launch_bounds__(256) accum_int_kernel(const float* __restrict_
     acc[(size_t)j * anx + i] += sum;
 }
 
+// acc += the sampled pass's group sums, in group order
+__global__ void __launch_bounds__(256) accum_parts_kernel(const double* __restrict__ part, int groups, long long n,
+                                                          double* __restrict__ acc)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double s = 0.;
+    for (int g = 0; g < groups; g++) s += part[g * n + i];
+    acc[i] += s;
+}
+
 // magnitude^2 of the n complex values at float2 offset `off` of the plan's tables when all of them
 // have it (relative spread within 1e-6), else -1
 static double flat_mag2(const std::vector<float2>& T, long long off, int n)
@@ -143,7 +144,12 @@ static double flat_mag2(const std::vector<float2>& T, long long off, int n)
 // sample instead of two complex values).  Where its output factors -- the output chain's table along
 // the lines and every chain's line factor -- have one magnitude, |f v|^2 = |f|^2 |v|^2: the pass
 // skips them and scales the intensity by that magnitude squared.
-static void mark_intensity_pass(std::vector<KernelDesc>& ks, const std::vector<float2>& tables)
+// Along the rows, where a detector row (azStep apart, anx columns) lies two output rows (zStep) or more
+// from the next, only the two rows around each are transformed, in one pass with the accumulation
+// (out_int 2): 2 zStep / azStep of the rows, and no intensities written and read back.  Closer detector rows would
+// transform rows twice: all rows then, once (out_int 1).
+static void mark_intensity_pass(std::vector<KernelDesc>& ks, const std::vector<float2>& tables, int anx, double azStep,
+                                double zStep)
 {
     for (size_t i = ks.size(); i-- > 0;) {
         if (reads_only(ks[i].kind)) continue;
@@ -155,6 +161,17 @@ static void mark_intensity_pass(std::vector<KernelDesc>& ks, const std::vector<f
                 // a column pass writes the intensity in blocks of its tile's columns (contiguous
                 // pieces); the accumulation reads that layout
                 if (d.axis == 1 && d.blk_out == 0) d.blk_out = pair_block(N, d.nx);
+                LineLaunch shape;
+                memset(&shape, 0, sizeof(shape));
+                if (d.axis == 0 && azStep >= 2. * std::fabs(zStep) && line_config(d, shape) == 0 && sample_fits(shape, anx)) {
+                    d.out_int = 2;
+                    // single rows are read, not blocks of them: row-major before this pass
+                    if (d.blk_in > 0 && i > 0 && ks[i - 1].kind == K_LINE) {
+                        d.blk_in = 0;
+                        ks[i - 1].line.blk_out = 0;
+                        fill_line_run(ks[i - 1].line);
+                    }
+                }
                 const ChainTab& out = d.f1 ? d.t_mid : d.t_fin;
                 const double a = flat_mag2(tables, out.tab, N), b = flat_mag2(tables, d.t_pre.ltab, nl),
                              c = flat_mag2(tables, d.t_mid.ltab, nl), e = flat_mag2(tables, d.t_fin.ltab, nl);
@@ -169,15 +186,17 @@ static void mark_intensity_pass(std::vector<KernelDesc>& ks, const std::vector<f
     }
 }
 
-static bool intensity_pass(const std::vector<KernelDesc>& ks, int* bw = nullptr)
+// whether the last pass writes the intensity (1) or adds it to the detector's sums itself (2); bw: the width of
+// the column blocks it is written in
+static int intensity_pass(const std::vector<KernelDesc>& ks, int* bw = nullptr)
 {
     for (size_t i = ks.size(); i-- > 0;)
         if (!reads_only(ks[i].kind)) {
-            const bool yes = ks[i].kind == K_LINE && ks[i].line.out_int;
+            const int yes = ks[i].kind == K_LINE ? ks[i].line.out_int : 0;
             if (bw) *bw = yes && ks[i].line.axis == 1 ? ks[i].line.blk_out : 0;
             return yes;
         }
-    return false;
+    return 0;
 }
 
 }  // namespace srwg
@@ -204,8 +223,13 @@ struct srwgMultiE {
     // batch buffers
     int maxBatch = 0;
     size_t nIn = 0, nOut = 0, perWork = 0, constStride = 0, descOff = 0;
-    float2* dOut = nullptr;              // [2][B][nOut]
-    float2* dWork = nullptr;             // [4][B][perWork]
+    int sub = 0;                         // a batch runs `sub` electrons at a time through all passes
+    float2* dOut = nullptr;              // fields [2][sub][nOut] or intensities [sub][nOut], when written
+    size_t outBytes = 0;
+    float2* dWork = nullptr;             // [4][sub][perWork]
+    double* dPart = nullptr;             // sampled last pass: sums of its groups of electrons [groups][anz][anx]
+    int parts = 0;                       // groups per sub-batch at most
+    int timedSubs = 0;                   // sub-batches of the last timed batch
     // per-electron constants (tables, descriptors) and parameters in two slots used in turn: the
     // host stages batch k+1 in pinned memory and a copy stream uploads it while batch k runs
     char* dConst[2] = {nullptr, nullptr};          // [B][constStride] per slot
@@ -232,7 +256,7 @@ struct srwgMultiE {
             if (graph[i]) cudaGraphExecDestroy(graph[i]);
         if (ownAcc) cudaFree(dAcc);
         cudaFree(dSnap);
-        cudaFree(dBase); cudaFree(dOut); cudaFree(dWork);
+        cudaFree(dBase); cudaFree(dOut); cudaFree(dWork); cudaFree(dPart);
         for (int i = 0; i < 2; i++) {
             cudaFree(dConst[i]);
             cudaFree(dParams[i]);
@@ -311,31 +335,96 @@ static bool same_structure(const std::vector<KernelDesc>& a, const std::vector<K
     return true;
 }
 
-// runs one batch: passes (the first one applies each electron's kick) -> accumulation; ks = launch
-// shapes (largest resize tiles of the batch)
+// device memory for what the last pass writes and the sampled pass's sums (made before a capture: every
+// launch sequence runs once directly first)
+static int ensure_out(srwgMultiE& m, int inten)
+{
+    const size_t need = inten == 2 ? 0 : (size_t)m.sub * m.nOut * (inten ? sizeof(float) : 2 * sizeof(float2));
+    if (need > m.outBytes) {
+        cudaFree(m.dOut);
+        m.dOut = nullptr;
+        m.outBytes = 0;
+        MTRY(cudaMalloc(&m.dOut, need));
+        m.outBytes = need;
+    }
+    if (inten == 2 && m.dPart == nullptr) {
+        // about 1500 CTAs of one detector row each
+        m.parts = std::min(m.sub, 1500 / m.anz + 1);
+        MTRY(cudaMalloc(&m.dPart, (size_t)m.parts * m.anx * m.anz * sizeof(double)));
+    }
+    return 0;
+}
+
+// runs one batch, a sub-batch after the other: passes (the first one applies each electron's kick) ->
+// accumulation; ks = launch shapes (largest resize tiles, widest windows)
 static int run_batch(srwgMultiE& m, int nb, const std::vector<KernelDesc>& ks, cudaStream_t st, int slot)
 {
     dim3 blk(256);
-    float2* outX = m.dOut;
-    float2* outY = m.dOut + (size_t)m.maxBatch * m.nOut;
     if (ks.empty()) { set_last_detail("multi-electron plan without passes"); return SRWG_ERR_BAD_ARG; }
-    // every electron's first pass reads the base field (input stride 0) and applies its kick
-    cudaEvent_t* ev = m.tev.size() >= 2 * ks.size() + 2 ? m.tev.data() : nullptr;
-    int r = execute_passes(ks, *m.ctx, nb, m.dBase, m.dBase + m.nIn, 0, outX, outY, (long long)m.nOut, m.dWork,
-                           m.perWork, m.dConst[slot], (long long)m.constStride, m.descOff, st, ev, &ks);
-    if (r) return r;
-    dim3 ga((m.anx + 255) / 256, m.anz);
-    if (ev) MTRY(cudaEventRecord(ev[2 * ks.size()], st));
     int bw = 0;
-    if (intensity_pass(ks, &bw))
-        accum_int_kernel<<<bw > 0 ? dim3((m.anz + 255) / 256, m.anx) : ga, blk, 0, st>>>(
-            reinterpret_cast<const float*>(outX), (long long)m.nOut, nb, m.dParams[slot],
-                                             m.dAcc, m.anx, m.anz, m.axStart, m.axStep, m.azStart, m.azStep, bw);
-    else
-        accum_kernel<<<ga, blk, 0, st>>>(outX, outY, (long long)m.nOut, nb, m.dParams[slot], m.dAcc, m.anx, m.anz,
-                                         m.axStart, m.axStep, m.azStart, m.azStep);
-    MTRY(cudaGetLastError());
-    if (ev) MTRY(cudaEventRecord(ev[2 * ks.size() + 1], st));
+    const int inten = intensity_pass(ks, &bw);
+    int r = ensure_out(m, inten);
+    if (r) return r;
+    const size_t nk = ks.size(), ne = 2 * nk + 2;
+    m.timedSubs = 0;
+    for (int b0 = 0; b0 < nb; b0 += m.sub) {
+        const int n = std::min(m.sub, nb - b0);
+        float2* outX = m.dOut;
+        float2* outY = m.dOut + (inten ? 0 : (size_t)m.sub * m.nOut);
+        const char* dc = m.dConst[slot] + (size_t)b0 * m.constStride;
+        const ElecParams* ep = m.dParams[slot] + b0;
+        cudaEvent_t* ev = m.tev.size() >= ne * (m.timedSubs + 1) ? m.tev.data() + ne * m.timedSubs : nullptr;
+        m.timedSubs++;
+        // every electron's first pass reads the base field (input stride 0) and applies its kick
+        r = execute_passes(ks, *m.ctx, n, m.dBase, m.dBase + m.nIn, 0, outX, outY, (long long)m.nOut, m.dWork, m.perWork, dc,
+                           (long long)m.constStride, m.descOff, st, ev, &ks, nullptr, nullptr, 0, nullptr,
+                           inten == 2 ? nk - 1 : nk);
+        if (r) return r;
+        if (inten == 2) {
+            const KernelDesc& k = ks[nk - 1];
+            LineLaunch p;
+            memset(&p, 0, sizeof(p));
+            p.nb = n;
+            r = line_config(k.line, p);
+            if (r) return r;
+            r = device_twiddles(*m.ctx, p.N, &p.tw);
+            if (r) return r;
+            const size_t W = (size_t)n * m.perWork;
+            const bool fromIn = k.src == 0;
+            p.src[0] = fromIn ? m.dBase : m.dWork + (k.src == 1 ? 0 : 2) * W;
+            p.src[1] = fromIn ? m.dBase + m.nIn : p.src[0] + W;
+            p.tabs = (const float2*)dc;
+            p.gd = &((const KernelDesc*)(dc + m.descOff))[nk - 1].line;
+            p.bDesc = (long long)m.constStride;
+            p.bTab = (long long)(m.constStride / sizeof(float2));
+            p.bSrc = fromIn ? 0 : (long long)m.perWork;
+            SampleArgs q;
+            q.ep = ep;
+            q.part = m.dPart;
+            q.nb = n;
+            q.per = (n + m.parts - 1) / m.parts;
+            q.anx = m.anx; q.anz = m.anz;
+            q.axStart = m.axStart; q.axStep = m.axStep; q.azStart = m.azStart; q.azStep = m.azStep;
+            if (ev) MTRY(cudaEventRecord(ev[2 * (nk - 1)], st));
+            MTRY(launch_line_sample(p, q, st, nk > 1 && ev == nullptr));
+            if (ev) MTRY(cudaEventRecord(ev[2 * (nk - 1) + 1], st));
+            if (ev) MTRY(cudaEventRecord(ev[2 * nk], st));
+            const long long na = (long long)m.anx * m.anz;
+            accum_parts_kernel<<<(unsigned)((na + 255) / 256), blk, 0, st>>>(m.dPart, (n + q.per - 1) / q.per, na, m.dAcc);
+        } else {
+            const dim3 ga((m.anx + 255) / 256, m.anz);
+            if (ev) MTRY(cudaEventRecord(ev[2 * nk], st));
+            if (inten)
+                accum_int_kernel<<<bw > 0 ? dim3((m.anz + 255) / 256, m.anx) : ga, blk, 0, st>>>(
+                    reinterpret_cast<const float*>(outX), (long long)m.nOut, n, ep, m.dAcc, m.anx, m.anz, m.axStart, m.axStep,
+                    m.azStart, m.azStep, bw);
+            else
+                accum_kernel<<<ga, blk, 0, st>>>(outX, outY, (long long)m.nOut, n, ep, m.dAcc, m.anx, m.anz, m.axStart,
+                                                 m.axStep, m.azStart, m.azStep);
+        }
+        MTRY(cudaGetLastError());
+        if (ev) MTRY(cudaEventRecord(ev[2 * nk + 1], st));
+    }
     return 0;
 }
 
@@ -378,55 +467,39 @@ static int flush(srwgMultiE& m, int nb, std::vector<KernelDesc>& ks, cudaStream_
         for (size_t i = 0; fits && i < ks.size(); i++) {
             const KernelDesc &a = ks[i], &g = m.graphKs[s][i];
             if (a.kind == K_RESIZE &&
-                (a.rs.tile_or > g.rs.tile_or || a.rs.tile_oc > g.rs.tile_oc || a.rs.ixStart < g.rs.ixStart ||
-                 a.rs.ixEnd > g.rs.ixEnd || a.rs.izStart < g.rs.izStart || a.rs.izEnd > g.rs.izEnd))
+                (a.rs.tile_or > g.rs.tile_or || a.rs.tile_oc > g.rs.tile_oc || a.rs.ixEnd > g.rs.ixEnd ||
+                 a.rs.izEnd > g.rs.izEnd))
                 fits = false;
-            if (a.kind == K_LINE && a.line.zwin && (a.line.zl0 < g.line.zl0 || a.line.zl1 > g.line.zl1)) fits = false;
+            if (a.kind == K_LINE && a.line.zwin && a.line.zl1 > g.line.zl1) fits = false;
         }
         if (!fits) {
-            // the new graph's shapes cover this batch, the graph it replaces (so that the windows
-            // grow to what the electrons' distribution needs in a few captures; an instantiation
-            // costs milliseconds of host time) and headroom for other batches: larger tiles,
-            // windows wider by a quarter of theirs (every CTA launched outside an electron's window
-            // costs a little)
+            // the new graph's shapes cover this batch, the graph it replaces and a little more (tiles of
+            // the resize, a line block or two of window), so that batches seldom need another one: an
+            // instantiation costs milliseconds of host time
             std::vector<KernelDesc> cap = ks;
-            if (m.graph[s] && m.graphKs[s].size() == cap.size())
-                for (size_t i = 0; i < cap.size(); i++) {
-                    const KernelDesc& o = m.graphKs[s][i];
-                    if (cap[i].kind == K_RESIZE) {
-                        ResizeDesc& r = cap[i].rs;
-                        r.tile_or = std::max(r.tile_or, o.rs.tile_or);
-                        r.tile_oc = std::max(r.tile_oc, o.rs.tile_oc);
-                        r.ixStart = std::min(r.ixStart, o.rs.ixStart);
-                        r.ixEnd = std::max(r.ixEnd, o.rs.ixEnd);
-                        r.izStart = std::min(r.izStart, o.rs.izStart);
-                        r.izEnd = std::max(r.izEnd, o.rs.izEnd);
-                    } else if (cap[i].kind == K_LINE && cap[i].line.zwin) {
-                        cap[i].line.zl0 = std::min(cap[i].line.zl0, o.line.zl0);
-                        cap[i].line.zl1 = std::max(cap[i].line.zl1, o.line.zl1);
-                    }
-                }
-            if (m.graph[s]) { cudaGraphExecDestroy(m.graph[s]); m.graph[s] = nullptr; }
+            const bool had = m.graph[s] && m.graphKs[s].size() == cap.size();
             for (size_t i = 0; i < cap.size(); i++) {
-                if (cap[i].kind == K_RESIZE && cap[i].rs.tile_or > 0) {
+                if (cap[i].kind == K_RESIZE) {
                     ResizeDesc& r = cap[i].rs;
-                    r.tile_or = std::min(SRWG_RESIZE_OR_MAX, r.tile_or + 2);
-                    r.tile_oc = std::min(SRWG_RESIZE_OC_MAX, r.tile_oc + 2);
-                    const long mx = std::max(2L * SRWG_RESIZE_TX, (r.ixEnd - r.ixStart) / 4);
-                    const long mz = std::max(2L * SRWG_RESIZE_TZ, (r.izEnd - r.izStart) / 4);
-                    r.ixStart = std::max(0L, r.ixStart - mx);
-                    r.ixEnd = std::min((long)r.nxn - 1, r.ixEnd + mx);
-                    r.izStart = std::max(0L, r.izStart - mz);
-                    r.izEnd = std::min((long)r.nzn - 1, r.izEnd + mz);
-                }
-                if (cap[i].kind == K_LINE && cap[i].line.zwin) {
-                    LineDesc& d = cap[i].line;
-                    const int nl = d.axis == 0 ? d.nz : d.nx;
-                    const int ml = std::max(64, (d.zl1 - d.zl0) / 4);
-                    d.zl0 = std::max(0, d.zl0 - ml);
-                    d.zl1 = std::min(nl - 1, d.zl1 + ml);
+                    if (r.tile_or > 0) {
+                        r.tile_or = std::min(SRWG_RESIZE_OR_MAX, r.tile_or + 2);
+                        r.tile_oc = std::min(SRWG_RESIZE_OC_MAX, r.tile_oc + 2);
+                    }
+                    r.ixEnd += 8;
+                    r.izEnd += 8;
+                    if (had) {
+                        const ResizeDesc& o = m.graphKs[s][i].rs;
+                        r.tile_or = std::max(r.tile_or, o.tile_or);
+                        r.tile_oc = std::max(r.tile_oc, o.tile_oc);
+                        r.ixEnd = std::max(r.ixEnd, o.ixEnd);
+                        r.izEnd = std::max(r.izEnd, o.izEnd);
+                    }
+                } else if (cap[i].kind == K_LINE && cap[i].line.zwin) {
+                    cap[i].line.zl1 += 8;
+                    if (had) cap[i].line.zl1 = std::max(cap[i].line.zl1, m.graphKs[s][i].line.zl1);
                 }
             }
+            if (m.graph[s]) { cudaGraphExecDestroy(m.graph[s]); m.graph[s] = nullptr; }
             // this batch runs directly (which also creates every lazily made resource -- twiddle
             // tables, kernel attributes -- before the capture); the capture only records the launches
             r = run_batch(m, nb, cap, st, s);
@@ -457,6 +530,16 @@ static int flush(srwgMultiE& m, int nb, std::vector<KernelDesc>& ks, cudaStream_
 }
 
 }  // namespace srwg
+
+// electrons that run through the passes together: a whole batch while its work buffers (perWork points
+// in four of them) stay within 8 GiB, else equal parts.  (Smaller parts, whose fields would stay in the L2
+// cache from pass to pass, measured no faster: 64 wavefronts at 1536 x 1600 1254 us whole, 1271 in two
+// parts, 1259 in four, 1343 in eight.)
+static int sub_batch(size_t perWork, int maxBatch)
+{
+    const size_t parts = ((size_t)maxBatch * 4 * perWork * sizeof(float2) + ((size_t)8 << 30) - 1) / ((size_t)8 << 30);
+    return (int)((maxBatch + parts - 1) / std::max<size_t>(parts, 1));
+}
 
 extern "C" SRWG_API int srwgMultiECreate(const SRWLWfr* pBase, const SRWLOptC* pOpt, const SRWLRadMesh* pAccMesh,
                                          int maxBatch, int useGraph, int device, srwgMultiE** out)
@@ -498,7 +581,7 @@ extern "C" SRWG_API int srwgMultiECreate(const SRWLWfr* pBase, const SRWLOptC* p
     pl.numMoments = false;               // only the intensity is kept: no moment passes
     pl.inPhase = true;                   // the electrons' kick (here zero): the same passes as theirs
     r = pl.plan(pBase, pOpt);
-    if (!r) mark_intensity_pass(pl.kernels, pl.tables);
+    if (!r) mark_intensity_pass(pl.kernels, pl.tables, m->anx, m->azStep, pl.w.zStep);
     if (r) { set_last_detail(pl.err); delete m; return r; }
     m->nIn = (size_t)m->nx * m->nz;
     m->nOut = (size_t)pl.w.nx * pl.w.nz;
@@ -517,9 +600,9 @@ extern "C" SRWG_API int srwgMultiECreate(const SRWLWfr* pBase, const SRWLOptC* p
         }                                                                            \
     } while (0)
     const size_t B = (size_t)maxBatch;
+    m->sub = sub_batch(m->perWork, maxBatch);
     MALLOC(m->dBase, 2 * m->nIn * sizeof(float2));
-    MALLOC(m->dOut, 2 * B * m->nOut * sizeof(float2));
-    MALLOC(m->dWork, 4 * B * m->perWork * sizeof(float2));
+    MALLOC(m->dWork, 4 * (size_t)m->sub * m->perWork * sizeof(float2));
     for (int i = 0; i < 2; i++) {
         MALLOC(m->dConst[i], B * m->constStride);
         MALLOC(m->dParams[i], B * sizeof(ElecParams));
@@ -551,6 +634,8 @@ extern "C" SRWG_API int srwgMultiECreate(const SRWLWfr* pBase, const SRWLOptC* p
         delete m;
         return SRWG_ERR_CUDA;
     }
+    r = ensure_out(*m, intensity_pass(pl.kernels));
+    if (r) { delete m; return MEMORY_ALLOCATION_FAILURE; }
     m->base.arEx = nullptr;           // the host arrays are not kept
     m->base.arEy = nullptr;
     *out = m;
@@ -587,7 +672,7 @@ extern "C" SRWG_API int srwgMultiEAddTimed(srwgMultiE* m, int n, const double* a
         pl.inPhase = true;
         r = pl.plan(&m->base, m->opt);
         if (r) { set_last_detail(pl.err); return r; }
-        const size_t ne = 2 * pl.kernels.size() + 2;
+        const size_t ne = (2 * pl.kernels.size() + 2) * (size_t)((m->maxBatch + m->sub - 1) / m->sub);
         for (cudaEvent_t e : m->tev) cudaEventDestroy(e);
         m->tev.assign(ne, nullptr);
         for (size_t i = 0; i < ne; i++) MTRY(cudaEventCreate(&m->tev[i]));
@@ -599,15 +684,20 @@ extern "C" SRWG_API int srwgMultiEAddTimed(srwgMultiE* m, int n, const double* a
         set_last_detail("timed add: the electrons did not run as one batch");
         r = SRWG_ERR_BAD_ARG;
     }
-    const int np = (int)(m->tev.size() / 2);
+    // (summed over the sub-batches)
+    const int np = (int)(m->tev.size() / 2 / (size_t)((m->maxBatch + m->sub - 1) / m->sub));
     if (r == 0) {
         DeviceCtx* c = nullptr;
         r = device_ctx(m->device, &c);
         if (r == 0 && cudaStreamSynchronize(stream ? (cudaStream_t)stream : c->stream) != cudaSuccess) r = SRWG_ERR_CUDA;
         for (int i = 0; r == 0 && i < np && i < maxPasses; i++) {
-            float ms = 0.f;
-            if (cudaEventElapsedTime(&ms, m->tev[2 * i], m->tev[2 * i + 1]) != cudaSuccess) r = SRWG_ERR_CUDA;
-            passMs[i] = ms;
+            passMs[i] = 0.f;
+            for (int s = 0; s < m->timedSubs; s++) {
+                float ms = 0.f;
+                const size_t o = 2 * (size_t)(s * np + i);
+                if (cudaEventElapsedTime(&ms, m->tev[o], m->tev[o + 1]) != cudaSuccess) r = SRWG_ERR_CUDA;
+                passMs[i] += ms;
+            }
         }
         if (nPasses) *nPasses = np;
     }
@@ -703,7 +793,7 @@ static int add_body(srwgMultiE* m, int n, const double* arOffsets, int stride, c
                     pls[k].inKz = eps[k].kz;
                     pls[k].inC = -(eps[k].kx * eps[k].dx + eps[k].kz * eps[k].dz);
                     rcs[k] = pls[k].plan(&w, m->opt);
-                    if (!rcs[k]) mark_intensity_pass(pls[k].kernels, pls[k].tables);
+                    if (!rcs[k]) mark_intensity_pass(pls[k].kernels, pls[k].tables, m->anx, m->azStep, pls[k].w.zStep);
                 }
             };
             m->pool->run(std::min(nthr, cnt), work);
@@ -725,21 +815,26 @@ static int add_body(srwgMultiE* m, int n, const double* arOffsets, int stride, c
             nb = 0;
         }
         if (nb == 0) { first = pl.kernels; launchKs = pl.kernels; }
-        // launch shapes of the batch: the largest resize tiles and the union of the windows (the
-        // kernels read every electron's own descriptor)
+        // launch shapes of the batch: the largest resize tiles and the widest windows, as windows from 0
+        // (the kernels read every electron's own descriptor)
+        const bool firstOne = nb == 0;
         for (size_t i = 0; i < launchKs.size(); i++)
             if (launchKs[i].kind == K_RESIZE) {
                 ResizeDesc &a = launchKs[i].rs;
                 const ResizeDesc& b = pl.kernels[i].rs;
+                const long wx = b.ixEnd - b.ixStart, wz = b.izEnd - b.izStart;
                 a.tile_or = std::max(a.tile_or, b.tile_or);
                 a.tile_oc = std::max(a.tile_oc, b.tile_oc);
-                a.ixStart = std::min(a.ixStart, b.ixStart);
-                a.ixEnd = std::max(a.ixEnd, b.ixEnd);
-                a.izStart = std::min(a.izStart, b.izStart);
-                a.izEnd = std::max(a.izEnd, b.izEnd);
+                a.ixEnd = firstOne ? wx : std::max(a.ixEnd, wx);
+                a.izEnd = firstOne ? wz : std::max(a.izEnd, wz);
+                a.ixStart = a.izStart = 0;
             } else if (launchKs[i].kind == K_LINE && launchKs[i].line.zwin) {
-                launchKs[i].line.zl0 = std::min(launchKs[i].line.zl0, pl.kernels[i].line.zl0);
-                launchKs[i].line.zl1 = std::max(launchKs[i].line.zl1, pl.kernels[i].line.zl1);
+                LineDesc& a = launchKs[i].line;
+                const LineDesc& b = pl.kernels[i].line;
+                const int w = b.zl1 - b.zl0, n = b.za1 - b.za0;
+                a.zl1 = firstOne ? w : std::max(a.zl1, w);
+                a.za1 = firstOne ? n : std::max(a.za1, n);
+                a.zl0 = a.za0 = 0;
             }
         pending.emplace_back(g, nb);
         // output mesh as the reference's SRWLWfr holds it, step re-derived from (Fin - Start)/(n - 1)
@@ -771,7 +866,7 @@ extern "C" SRWG_API int srwgMultiEInfo(srwgMultiE* m, int* nPasses, int* intensi
     pl.inPhase = true;
     int r = pl.plan(&m->base, m->opt);
     if (r) { set_last_detail(pl.err); return r; }
-    mark_intensity_pass(pl.kernels, pl.tables);
+    mark_intensity_pass(pl.kernels, pl.tables, m->anx, m->azStep, pl.w.zStep);
     if (nPasses) *nPasses = (int)pl.kernels.size();
     if (intensityPass) *intensityPass = intensity_pass(pl.kernels) ? 1 : 0;
     if (desc && descLen > 0) {

@@ -1772,6 +1772,10 @@ void fill_line_run(LineDesc& d)
     r.mirror_lines = d.mirror_lines;
     r.zwin = d.zwin; r.zl0 = d.zl0; r.zl1 = d.zl1; r.za0 = d.za0; r.za1 = d.za1; r.zskip = d.zskip;
     r.blk_in = d.blk_in; r.blk_out = d.blk_out;
+    const int N = d.axis == 0 ? d.nx : d.nz, nl = d.axis == 0 ? d.nz : d.nx;
+    r.in_p = d.in_p ? d.in_p : (d.blk_in > 0 || d.axis == 0) ? N : nl;
+    r.out_p = d.out_p ? d.out_p : (d.blk_out > 0 || d.axis == 1) ? nl : N;
+    r.in_l0 = d.in_l0; r.in_q0 = d.in_q0; r.out_l0 = d.out_l0;
     r.extra = d.has_extra;
     r.int_flat = d.int_flat; r.int_scale = d.int_scale;
     r.ang = d.ang; r.qtab = d.qtab; r.qline = d.qline; r.qc0 = d.qc0; r.qc1 = d.qc1;
@@ -1847,6 +1851,15 @@ int Planner::finalize()
         d.zwin = 1;
         if (d.axis == 0) { d.zl0 = izs; d.zl1 = ize; d.za0 = ixs; d.za1 = ixe; }
         else { d.zl0 = ixs; d.zl1 = ixe; d.za0 = izs; d.za1 = ize; }
+        // only the window is stored (whole pairs of lines along either axis)
+        if (ixs <= ixe && izs <= ize) {
+            r.cx0 = ixs & ~1;
+            r.cz0 = izs & ~1;
+            r.cp = (ixe - r.cx0 + 2) & ~1;
+            d.in_p = r.cp;
+            d.in_l0 = d.axis == 0 ? r.cz0 : r.cx0;
+            d.in_q0 = d.axis == 0 ? r.cx0 : r.cz0;
+        }
     }
     // a row pass followed by a column pass on its output writes it in blocks of as many columns as
     // a column CTA transforms, so that the column pass reads whole blocks sequentially
@@ -1894,6 +1907,13 @@ int Planner::finalize()
         d.za0 = a.line.mirror_lines ? np - 1 - a.line.zl1 : a.line.zl0;
         d.za1 = a.line.mirror_lines ? np - 1 - a.line.zl0 : a.line.zl1;
         a.line.zskip = 1;
+        // only those lines are stored: rows whole, in columns and blocks side by side
+        if (d.za0 <= d.za1) {
+            a.line.out_l0 = d.in_q0 = d.za0 & ~1;
+            const int n1 = (d.za1 - a.line.out_l0 + 2) & ~1;
+            if (a.line.blk_out > 0 || a.line.axis == 1) a.line.out_p = n1;
+            if (d.blk_in > 0 || d.axis == 0) d.in_p = n1;
+        }
     }
     for (KernelDesc& k : kernels)
         if (k.kind == K_LINE) fill_line_run(k.line);
