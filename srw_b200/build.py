@@ -13,7 +13,7 @@ OBJ_DIR = os.path.join(HERE, '_build')          # objects: kept out of the shipp
 LIB = os.path.join(OUT_DIR, 'libsrwl_b200.so')
 NVCC = os.environ.get('NVCC', '/usr/local/cuda/bin/nvcc')
 ARCH = ['-gencode', 'arch=compute_100a,code=sm_100a']
-SOURCES = ['kernels.cu', 'line2_14.cu', 'line2e_14.cu', 'planner.cpp', 'tables.cpp', 'capi.cpp', 'noalloc.cu',
+SOURCES = ['kernels.cu', 'line2_14.cu', 'line2e_14.cu', 'planner.cpp', 'tables.cpp', 'capi.cpp', 'hostcopy.cpp', 'noalloc.cu',
            'multie.cu', 'mlp.cu', 'moments.cu', 'intensity.cu', 'gaussian.cu']
 # the line passes on pairs: a unit per (axis, mode) (csrc/linep.cu)
 LINEP = ['linep.cu@%d,%d' % (c, m) for c in (0, 1) for m in (0, 1, 2)]

@@ -629,6 +629,31 @@ int srwlUtiGetErrText(char* t, int erNo)
     return 0;
 }
 
+// the caller's field components into (dX, dY), zeros for one that is absent
+static int field_to_device(DeviceCtx& c, const SRWLWfr* w, size_t n, float2* dX, float2* dY, cudaStream_t st)
+{
+    CopySeg seg[2];
+    int k = 0;
+    if (w->arEx) seg[k++] = {w->arEx, dX, n * sizeof(float2)};
+    else CUDA_TRY(cudaMemsetAsync(dX, 0, n * sizeof(float2), st));
+    if (w->arEy) seg[k++] = {w->arEy, dY, n * sizeof(float2)};
+    else CUDA_TRY(cudaMemsetAsync(dY, 0, n * sizeof(float2), st));
+    CUDA_TRY(copy_segments(c.ring, c.dev, seg, k, true, st));
+    return 0;
+}
+
+// (dX, dY) into the caller's arrays, those that are there; the stream has finished on return
+static int field_to_host(DeviceCtx& c, char* hX, char* hY, size_t n, float2* dX, float2* dY, cudaStream_t st)
+{
+    CopySeg seg[2];
+    int k = 0;
+    if (hX) seg[k++] = {hX, dX, n * sizeof(float2)};
+    if (hY) seg[k++] = {hY, dY, n * sizeof(float2)};
+    CUDA_TRY(copy_segments(c.ring, c.dev, seg, k, false, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
+    return 0;
+}
+
 // the intensity extractions of a stage that ran: each into the caller's array (allocated through the
 // registered allocation function when the caller passed none, AllocExtIntArray srradstr.cpp:799),
 // with its mesh (GetIntMesh, srradstr.cpp:4140: the wavefront's x and y mesh, eStart kept)
@@ -669,10 +694,8 @@ static int propagate_staged(Planner& pl, SRWLWfr* pWfr, int dev, int pr, char** 
     const size_t nIn = (size_t)pl.in.nx * pl.in.nz;
     r = ensure_io(*c, nIn);
     if (r) return r;
-    if (pWfr->arEx) CUDA_TRY(cudaMemcpyAsync(c->io, pWfr->arEx, nIn * sizeof(float2), cudaMemcpyHostToDevice, st));
-    else CUDA_TRY(cudaMemsetAsync(c->io, 0, nIn * sizeof(float2), st));
-    if (pWfr->arEy) CUDA_TRY(cudaMemcpyAsync(c->io + c->ioElems, pWfr->arEy, nIn * sizeof(float2), cudaMemcpyHostToDevice, st));
-    else CUDA_TRY(cudaMemsetAsync(c->io + c->ioElems, 0, nIn * sizeof(float2), st));
+    r = field_to_device(*c, pWfr, nIn, c->io, c->io + c->ioElems, st);
+    if (r) return r;
     const float2* curX = c->io;
     const float2* curY = c->io + c->ioElems;
     float2 *oX = nullptr, *oY = nullptr;
@@ -735,9 +758,8 @@ static int propagate_staged(Planner& pl, SRWLWfr* pWfr, int dev, int pr, char** 
         if ((*g_modifFunc)(2, pWfr, 0)) return SRWL_WFR_EXT_MODIF_FAILED;
         out_wfr(pl, pWfr);
     }
-    if (hadX && pWfr->arEx) CUDA_TRY(cudaMemcpyAsync(pWfr->arEx, oX, nOut * sizeof(float2), cudaMemcpyDeviceToHost, st));
-    if (hadY && pWfr->arEy) CUDA_TRY(cudaMemcpyAsync(pWfr->arEy, oY, nOut * sizeof(float2), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    r = field_to_host(*c, hadX ? pWfr->arEx : nullptr, hadY ? pWfr->arEy : nullptr, nOut, oX, oY, st);
+    if (r) return r;
     out_moments(pl, pWfr, slots.empty() ? nullptr : slots.data());
     return 0;
 }
@@ -794,10 +816,8 @@ int srwlPropagElecField(SRWLWfr* pWfr, SRWLOptC* pOpt, int nInt, char** arID, SR
     float2* outX = c->io + 2 * c->ioElems;
     float2* outY = c->io + 3 * c->ioElems;
     cudaStream_t st = c->stream;
-    if (pWfr->arEx) CUDA_TRY(cudaMemcpyAsync(inX, pWfr->arEx, nIn * sizeof(float2), cudaMemcpyHostToDevice, st));
-    else CUDA_TRY(cudaMemsetAsync(inX, 0, nIn * sizeof(float2), st));
-    if (pWfr->arEy) CUDA_TRY(cudaMemcpyAsync(inY, pWfr->arEy, nIn * sizeof(float2), cudaMemcpyHostToDevice, st));
-    else CUDA_TRY(cudaMemsetAsync(inY, 0, nIn * sizeof(float2), st));
+    r = field_to_device(*c, pWfr, nIn, inX, inY, st);
+    if (r) return r;
     r = upload_tables(pl, &c->tab, &c->tabElems, st);
     if (r) return r;
     const size_t nSlotD = (size_t)pl.nMomSlots * SRWG_MOM_SLOT;
@@ -819,9 +839,8 @@ int srwlPropagElecField(SRWLWfr* pWfr, SRWLOptC* pOpt, int nInt, char** arID, SR
         if ((*g_modifFunc)(2, pWfr, 0)) return SRWL_WFR_EXT_MODIF_FAILED;
         out_wfr(pl, pWfr);
     }
-    if (hadX && pWfr->arEx) CUDA_TRY(cudaMemcpyAsync(pWfr->arEx, outX, nOut * sizeof(float2), cudaMemcpyDeviceToHost, st));
-    if (hadY && pWfr->arEy) CUDA_TRY(cudaMemcpyAsync(pWfr->arEy, outY, nOut * sizeof(float2), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    r = field_to_host(*c, hadX ? pWfr->arEx : nullptr, hadY ? pWfr->arEy : nullptr, nOut, outX, outY, st);
+    if (r) return r;
     out_moments(pl, pWfr, nSlotD ? hs.data() : nullptr);
     return 0;
 }

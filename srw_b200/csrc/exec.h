@@ -4,6 +4,7 @@
 #include <mutex>
 #include <string>
 #include <vector>
+#include "hostcopy.h"
 #include "kernels.h"
 
 namespace srwg {
@@ -25,6 +26,7 @@ struct DeviceCtx {
     void* genBuf = nullptr;             // field generation: both components, tables, moment scratch
     size_t genBytes = 0;
     size_t stgElems[2] = {0, 0};
+    HostRing ring;                      // pinned blocks of the host-memory entry point's copies
     cudaStream_t stream = nullptr;
     int* status = nullptr;              // device counter of bounded waits that gave up (kernels add to it)
 };
