@@ -168,19 +168,42 @@ inline double radix_cost(int R)
 }
 const double STAGE_COST = 14.;           // twiddles and the exchange, per point
 
-// the cheapest product of radices (non-increasing) for N
-inline void best_radices(int N, int most, std::vector<int>& cur, double cost, std::vector<int>& best, double& bestCost)
+// The schedule of least cost: radices, and threads per pair.  A stage takes its rounds (butterflies per
+// thread) times a butterfly's instructions, and a constant for the barrier and its loads; a pair's threads
+// weigh by T^alpha.  Long lines fill the chip and the work counts (alpha = 1: no idle threads); short ones
+// are a chain of single warps that run every instruction once (at 216 x 200 ncu shows 8 of 13 cycles per
+// instruction waiting for code), so butterflies are small and threads many.  Propagations between drifts,
+// the work alone (radices 16 first, about 16 points per thread) and this rule: 100 x 90 55 and 45 us,
+// 216 x 200 57 and 45, 360 x 350 96 and 55, 500 x 504 64 and 59, 1000 x 1080 120 and 111, 1400 x 1470 222
+// and 206; 720 x 700 84 and 88; above 1600 points the work alone: 2000 x 1980 380, with alpha 0.7 403.
+inline void best_schedule(int N, int most, std::vector<int>& cur, std::vector<int>& best, int& bestT, double& bestCost)
 {
-    if (N == 1) {
-        if (cur.size() >= 2 && cost < bestCost) { bestCost = cost; best = cur; }
+    int m = N;
+    for (int R : cur) m /= R;
+    if (m == 1) {
+        if (cur.size() < 2) return;
+        // the first radix is even and, where there is one, at least 8 (neighbouring k1 then fill the banks)
+        size_t f = 0;
+        while (f < cur.size() && (cur[f] & 1)) f++;
+        if (f == cur.size()) return;
+        const double al = N <= 400 ? 0.3 : N <= 1600 ? 0.7 : 1., sy = N <= 400 ? 60. : 20.;
+        for (int T = std::max(1, N / 32); T <= std::min(512, std::max(1, N / 2)); T++) {
+            double w = 0.;
+            for (int R : cur) w += (double)((N / R + T - 1) / T) * (radix_cost(R) + STAGE_COST) * R + sy;
+            const double q = w * std::pow((double)T, al);
+            if (q < bestCost) {
+                bestCost = q;
+                bestT = T;
+                best = cur;
+                std::rotate(best.begin(), best.begin() + f, best.begin() + f + 1);
+            }
+        }
         return;
     }
     for (int R = std::min(most, 16); R >= 2; R--) {
-        if (N % R || (int)cur.size() + 1 > SRWG_MAX_STAGES) continue;
-        const double c = cost + radix_cost(R) + STAGE_COST;
-        if (c >= bestCost) continue;
+        if (m % R || (int)cur.size() + 1 > SRWG_MAX_STAGES) continue;
         cur.push_back(R);
-        best_radices(N / R, R, cur, c, best, bestCost);
+        best_schedule(N, R, cur, best, bestT, bestCost);
         cur.pop_back();
     }
 }
@@ -207,12 +230,8 @@ inline bool make_pair_shape(int N, PairShape& z)
 #undef SRWG_LINEF_SHAPE
     if (r.empty()) {
         double c = 1e300;
-        best_radices(N, 16, cur, 0., r, c);
+        best_schedule(N, 16, cur, r, z.T, c);
         if (r.empty()) return false;
-        // the first radix is even and, where there is one, at least 8 (neighbouring k1 then fill the banks)
-        size_t f = 0;
-        while (r[f] & 1) f++;
-        std::rotate(r.begin(), r.begin() + f, r.begin() + f + 1);
     }
     z.n = (int)r.size();
     z.len[0] = N;
@@ -234,21 +253,6 @@ inline bool make_pair_shape(int N, PairShape& z)
     for (int s = z.n - 1; s >= 1; s--) { z.tw2[s] = o; o += tw_rows(z.R[s]) * (N / z.len[s]); }
     z.tw1[z.n - 1] = z.tw2[0] = o;              // (not used)
     z.twLen = o;
-    // threads: the count that leaves the fewest idle in the stages' last rounds, about 16 points each
-    if (z.T) return true;
-    double bestT = 1e300;
-    for (int T = std::max(1, N / 32); T <= std::min(512, std::max(1, N / 4)); T++) {
-        double w = 0., ideal = 0.;
-        for (int s = 0; s < z.n; s++) {
-            const int M = N / z.R[s];
-            const double k = (radix_cost(z.R[s]) + STAGE_COST) * z.R[s];
-            w += (double)((M + T - 1) / T) * T * k;
-            ideal += M * k;
-        }
-        const double ppt = (double)N / T;
-        const double q = w / ideal * (1. + 0.02 * std::fabs(std::log2(ppt / 14.)));
-        if (q < bestT) { bestT = q; z.T = T; }
-    }
     return true;
 }
 
