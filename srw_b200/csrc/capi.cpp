@@ -328,7 +328,7 @@ int execute_passes(const std::vector<KernelDesc>& ks, DeviceCtx& c, int nb, cons
                    long long inStride, float2* outX, float2* outY, long long outStride, float2* work, size_t workElems,
                    const char* dconst, long long constStride, size_t descOff, cudaStream_t st, cudaEvent_t* ev,
                    const std::vector<KernelDesc>* hostMax, double* momScratch, double* momSlots, int nSlots,
-                   char* intOut, size_t nRun)
+                   char* intOut, size_t nRun, const unsigned* mask, int maskWords)
 {
     const size_t nk = ks.size();
     const size_t W = (size_t)nb * workElems;
@@ -396,6 +396,10 @@ int execute_passes(const std::vector<KernelDesc>& ks, DeviceCtx& c, int nb, cons
             p.byValue = hostMax == nullptr;
             p.run = k.line.run;
             line_window(k.line, p);
+            if (mask != nullptr && i + 1 == std::min(nRun, nk)) {
+                p.mask = mask;
+                p.maskWords = maskWords;
+            }
             e = launch_line(p, st, pdlOk);
         } else if (k.kind == K_RESIZE) {
             ResizeLaunch p;

@@ -38,7 +38,9 @@ int execute_passes(const std::vector<KernelDesc>& ks, DeviceCtx& c, int nb, cons
                    long long inStride, float2* outX, float2* outY, long long outStride, float2* work, size_t workElems,
                    const char* dconst, long long constStride, size_t descOff, cudaStream_t st, cudaEvent_t* ev,
                    const std::vector<KernelDesc>* hostMax, double* momScratch = nullptr, double* momSlots = nullptr,
-                   int nSlots = 0, char* intOut = nullptr, size_t nRun = (size_t)-1);   // nRun: only the first passes
+                   int nSlots = 0, char* intOut = nullptr,
+                   size_t nRun = (size_t)-1,          // only the first passes
+                   const unsigned* mask = nullptr, int maskWords = 0);   // rows the last of them has to write
 int line_config(const LineDesc& d, LineLaunch& p);   // launch shape of a line pass (capi.cpp)
 void line_window(const LineDesc& d, LineLaunch& p);  // only the window's line blocks (zskip row passes)
 void resize_window(const ResizeDesc& r, ResizeLaunch& p);   // only the window's tiles (skip_zero)

@@ -64,6 +64,8 @@ struct LineArgs {
     int bulk;                // points of staging per component behind the slots (0: no bulk copies)
     int* status;             // device counter of waits that gave up (NULL: not recorded)
     long long spin;          // iteration limit of the bulk-copy wait
+    const unsigned* mask;    // columns before a sampled pass: a bit per output row that it reads (NULL: all are)
+    int maskWords;           // words of it per wavefront
     int nblk;                // line blocks launched, from the window's first one (0: all)
 };
 struct LineLaunch : LineArgs {
@@ -88,6 +90,15 @@ struct SampleArgs {
     int nb, per, anx, anz;
     double axStart, axStep, azStart, azStep;
 };
+#ifdef __CUDACC__
+// detector row j and the output row below it on an electron's mesh (its operations written out: the pass
+// and the mask of the rows it reads agree)
+__device__ __forceinline__ double sample_y(const SampleArgs& q, int j) { return __fma_rn((double)j, q.azStep, q.azStart); }
+__device__ __forceinline__ int sample_row(const SampleArgs& q, const ElecParams& e, int j)
+{
+    return (int)trunc(__fma_rn(__dadd_rn(sample_y(q, j), -e.ozStart), e.ozInv, 1.e-09));
+}
+#endif
 
 // tiled resize: a CTA makes TZ x TX new points from an old tile of at most OR_MAX x OC_MAX points
 #define SRWG_RESIZE_TX 64
@@ -145,6 +156,8 @@ cudaError_t launch_extract(const MomDesc& d, const MomDesc* gd, const float2* s0
 // ends; it waits for it before it touches a field
 cudaError_t launch_line(const LineLaunch& p, cudaStream_t st, bool pdl = false);
 // the sampled row pass of a batch; its shape (threads, shared memory) must fit: sample_fits
+// the rows a sampled pass of descriptors p.gd reads, a bit each: words per electron, into mask
+cudaError_t launch_row_mask(const LineLaunch& p, const SampleArgs& q, unsigned* mask, int words, cudaStream_t st);
 cudaError_t launch_line_sample(const LineLaunch& p, const SampleArgs& q, cudaStream_t st, bool pdl);
 bool sample_fits(const LineLaunch& p, int anx);
 void fill_line_run(LineDesc& d);      // d.run from the rest of d (planner.cpp)

@@ -412,6 +412,7 @@ struct PLine {
     const PwOps* ex;
     int line0, line1;
     float* si;              // intensity line in shared memory
+    const unsigned* mask;   // columns: a bit per output point that is read (NULL: all of them are)
     bool has_lf;
     float2 lfr, lfi;        // line factors
     const float* qtab;      // quartic angular term (EXTRA 1): q^2 along the line, of the two lines, coefficients
@@ -565,16 +566,16 @@ __device__ __forceinline__ void pload(P2 (&v)[R], const PLine& x, const PChain& 
 
 // one output of both lines to p0 and p1; OUTI: the intensity of the pair (both components) as one float
 template <bool COLS, int OUTI>
-__device__ __forceinline__ void pput(const P2& o, const PLine& x, void* p0, float2* p1, float iscale)
+__device__ __forceinline__ void pput(const P2& o, const PLine& x, void* p0, float2* p1, float iscale, bool on = true)
 {
     if (OUTI) {
         const float2 I = __ffma2_rn(o.im, o.im, __fmul2_rn(o.re, o.re));
         if (x.st0) __stcs(reinterpret_cast<float*>(p0), (I.x + I.y) * iscale);
     } else if (COLS && x.vout) {
-        if (x.st0) __stcs(reinterpret_cast<float4*>(p0), make_float4(o.re.x, o.im.x, o.re.y, o.im.y));
+        if (x.st0 && on) __stcs(reinterpret_cast<float4*>(p0), make_float4(o.re.x, o.im.x, o.re.y, o.im.y));
     } else {
-        if (x.st0) __stcs(reinterpret_cast<float2*>(p0), make_float2(o.re.x, o.im.x));
-        if (x.st1) __stcs(p1, make_float2(o.re.y, o.im.y));
+        if (x.st0 && on) __stcs(reinterpret_cast<float2*>(p0), make_float2(o.re.x, o.im.x));
+        if (x.st1 && on) __stcs(p1, make_float2(o.re.y, o.im.y));
     }
 }
 
@@ -629,6 +630,15 @@ __device__ __forceinline__ void pstore(P2 (&v)[R], const PLine& x, const PChain&
         return;
     }
     constexpr int EB = OUTI ? 4 : 8;                     // bytes of an output element
+    auto wanted = [&](auto&& kk) {                       // bit r: point kk(r) is read
+        unsigned on = ~0u;
+        if (COLS && OUTI == 0 && x.mask != nullptr) {
+            on = 0;
+#pragma unroll
+            for (int r = 0; r < R; r++) on |= ((__ldg(x.mask + (kk(r) >> 5)) >> (kk(r) & 31)) & 1u) << r;
+        }
+        return on;
+    };
     const int h = c.rot_out ? (N >> 1) : 0;
     char* b0 = reinterpret_cast<char*>(x.o0);
     char* b1 = reinterpret_cast<char*>(x.o1);
@@ -647,22 +657,26 @@ __device__ __forceinline__ void pstore(P2 (&v)[R], const PLine& x, const PChain&
         const int kA = c.mir ? N - 1 - (u + h) : u + h, kB = c.mir ? N - 1 - (u - h) : u - h, ks = c.mir ? -M : M;
         const unsigned pA = x.ooff + (unsigned)x.place(kA), pB = x.ooff + (unsigned)x.place(kB);
         const unsigned ps = (unsigned)(x.lg < 0 ? ks * x.ostr : (ks >> x.lg) * x.bstr);
+        const unsigned on = wanted([&](int r) { return (r < R / 2 ? kA : kB) + r * ks; });
         pfactors<R, COLS, EXTRA>(v, x, c, N, [&](int r) { return (r < R / 2 ? kA : kB) + r * ks; });
 #pragma unroll
         for (int r = 0; r < R; r++) {
             const unsigned o = (r < R / 2 ? pA : pB) + (unsigned)r * ps;
-            pput<COLS, OUTI>(v[r], x, b0 + (size_t)o * EB, reinterpret_cast<float2*>(b1 + (size_t)o * EB), iscale);
+            pput<COLS, OUTI>(v[r], x, b0 + (size_t)o * EB, reinterpret_cast<float2*>(b1 + (size_t)o * EB), iscale,
+                             (on >> r) & 1u);
         }
     } else {
         auto kk = [&](int r) {
             const int k = prot(u + r * M, N, c.rot_out);
             return c.mir ? N - 1 - k : k;
         };
+        const unsigned on = wanted(kk);
         pfactors<R, COLS, EXTRA>(v, x, c, N, kk);
 #pragma unroll
         for (int r = 0; r < R; r++) {
             const unsigned o = x.ooff + (unsigned)x.place(kk(r));
-            pput<COLS, OUTI>(v[r], x, b0 + (size_t)o * EB, reinterpret_cast<float2*>(b1 + (size_t)o * EB), iscale);
+            pput<COLS, OUTI>(v[r], x, b0 + (size_t)o * EB, reinterpret_cast<float2*>(b1 + (size_t)o * EB), iscale,
+                             (on >> r) & 1u);
         }
     }
 }
@@ -921,6 +935,7 @@ __global__ void __launch_bounds__(512, 1) linep_kernel(const LineArgs p)
             x.vin = 0;
         }
     }
+    x.mask = COLS && p.mask != nullptr ? p.mask + blockIdx.z * p.maskWords : nullptr;
     x.tabs = p.tabs + blockIdx.z * p.bTab;
     x.ex = EXTRA == 2 ? &gd->extra : nullptr;
     PChain pre, mid, fin;
@@ -1048,7 +1063,6 @@ __global__ void __launch_bounds__(512, 1) linep_sample_kernel(const LineArgs p, 
     float* I1 = I0 + N;
     double* acc = reinterpret_cast<double*>(I0 + 2 * N + (N & 1) * 2);
     for (int i = tid; i < q.anx; i += blockDim.x) acc[i] = 0.;
-    const double y = q.azStart + (double)j * q.azStep;
     PLine x;
     x.g0 = x.g1 = nullptr;
     x.sg0 = x.sg1 = nullptr;
@@ -1063,7 +1077,8 @@ __global__ void __launch_bounds__(512, 1) linep_sample_kernel(const LineArgs p, 
     pdl_wait();
     for (int b = blockIdx.y * q.per; b < b1; b++) {
         const ElecParams& e = q.ep[b];
-        const int iy0 = (int)trunc((y - e.ozStart) * e.ozInv + 1.e-09);
+        const double y = sample_y(q, j);
+        const int iy0 = sample_row(q, e, j);
         if (iy0 < 0 || iy0 >= e.onz - 1) continue;
         const LineRun d = reinterpret_cast<const LineDesc*>(reinterpret_cast<const char*>(p.gd) + b * p.bDesc)->run;
         const int row = iy0 + g, line = d.mirror_lines ? nl - 1 - row : row;

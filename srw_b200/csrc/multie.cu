@@ -227,6 +227,7 @@ struct srwgMultiE {
     float2* dOut = nullptr;              // fields [2][sub][nOut] or intensities [sub][nOut], when written
     size_t outBytes = 0;
     float2* dWork = nullptr;             // [4][sub][perWork]
+    unsigned* dMask = nullptr;           // rows that the sampled last pass reads [electrons][words]
     double* dPart = nullptr;             // sampled last pass: sums of its groups of electrons [groups][anz][anx]
     int parts = 0;                       // groups per sub-batch at most
     int timedSubs = 0;                   // sub-batches of the last timed batch
@@ -256,7 +257,7 @@ struct srwgMultiE {
             if (graph[i]) cudaGraphExecDestroy(graph[i]);
         if (ownAcc) cudaFree(dAcc);
         cudaFree(dSnap);
-        cudaFree(dBase); cudaFree(dOut); cudaFree(dWork); cudaFree(dPart);
+        cudaFree(dBase); cudaFree(dOut); cudaFree(dWork); cudaFree(dPart); cudaFree(dMask);
         for (int i = 0; i < 2; i++) {
             cudaFree(dConst[i]);
             cudaFree(dParams[i]);
@@ -351,6 +352,7 @@ static int ensure_out(srwgMultiE& m, int inten)
         // about 1500 CTAs of one detector row each
         m.parts = std::min(m.sub, 1500 / m.anz + 1);
         MTRY(cudaMalloc(&m.dPart, (size_t)m.parts * m.anx * m.anz * sizeof(double)));
+        MTRY(cudaMalloc(&m.dMask, (size_t)m.sub * 256 * sizeof(unsigned)));
     }
     return 0;
 }
@@ -375,14 +377,12 @@ static int run_batch(srwgMultiE& m, int nb, const std::vector<KernelDesc>& ks, c
         const ElecParams* ep = m.dParams[slot] + b0;
         cudaEvent_t* ev = m.tev.size() >= ne * (m.timedSubs + 1) ? m.tev.data() + ne * m.timedSubs : nullptr;
         m.timedSubs++;
-        // every electron's first pass reads the base field (input stride 0) and applies its kick
-        r = execute_passes(ks, *m.ctx, n, m.dBase, m.dBase + m.nIn, 0, outX, outY, (long long)m.nOut, m.dWork, m.perWork, dc,
-                           (long long)m.constStride, m.descOff, st, ev, &ks, nullptr, nullptr, 0, nullptr,
-                           inten == 2 ? nk - 1 : nk);
-        if (r) return r;
+        LineLaunch p;
+        SampleArgs q;
+        const unsigned* mask = nullptr;
+        int words = 0;
         if (inten == 2) {
             const KernelDesc& k = ks[nk - 1];
-            LineLaunch p;
             memset(&p, 0, sizeof(p));
             p.nb = n;
             r = line_config(k.line, p);
@@ -398,13 +398,25 @@ static int run_batch(srwgMultiE& m, int nb, const std::vector<KernelDesc>& ks, c
             p.bDesc = (long long)m.constStride;
             p.bTab = (long long)(m.constStride / sizeof(float2));
             p.bSrc = fromIn ? 0 : (long long)m.perWork;
-            SampleArgs q;
             q.ep = ep;
             q.part = m.dPart;
             q.nb = n;
             q.per = (n + m.parts - 1) / m.parts;
             q.anx = m.anx; q.anz = m.anz;
             q.axStart = m.axStart; q.axStep = m.axStep; q.azStart = m.azStart; q.azStep = m.azStep;
+            // a column pass before it writes the rows that it reads
+            if (nk > 1 && ks[nk - 2].kind == K_LINE && ks[nk - 2].line.axis == 1 && pair_supported(ks[nk - 2].line.nz)) {
+                words = (p.nlines + 31) / 32;
+                MTRY(launch_row_mask(p, q, m.dMask, words, st));
+                mask = m.dMask;
+            }
+        }
+        // every electron's first pass reads the base field (input stride 0) and applies its kick
+        r = execute_passes(ks, *m.ctx, n, m.dBase, m.dBase + m.nIn, 0, outX, outY, (long long)m.nOut, m.dWork, m.perWork, dc,
+                           (long long)m.constStride, m.descOff, st, ev, &ks, nullptr, nullptr, 0, nullptr,
+                           inten == 2 ? nk - 1 : nk, mask, words);
+        if (r) return r;
+        if (inten == 2) {
             if (ev) MTRY(cudaEventRecord(ev[2 * (nk - 1)], st));
             MTRY(launch_line_sample(p, q, st, nk > 1 && ev == nullptr));
             if (ev) MTRY(cudaEventRecord(ev[2 * (nk - 1) + 1], st));
