@@ -813,7 +813,7 @@ __device__ __forceinline__ void run_back(const Z& z, float4* s, const PLine& x, 
 // MODE 0: one transform, 1: two transforms, 2: one transform and the intensity of both components.
 // Z: the length's schedule, fixed at compile time (FShape) or from the launch (PShape)
 template <class Z, bool COLS, int MODE, int EXTRA>
-__global__ void __launch_bounds__(512, 1) linep_kernel(const LineArgs p)
+__global__ void __launch_bounds__(Z::bound, 1) linep_kernel(const LineArgs p)
 {
     constexpr bool INT = MODE == 2;
     constexpr int LPP = INT ? 1 : 2;                     // lines per pair
@@ -1047,7 +1047,7 @@ __global__ void __launch_bounds__(512, 1) linep_kernel(const LineArgs p)
 // by accum_parts_kernel.  At 1536 x 1600 on 512^2 (a detector row per 5 output rows) it transforms 640 of
 // the 1600 rows and writes no intensities.
 template <class Z>
-__global__ void __launch_bounds__(512, 1) linep_sample_kernel(const LineArgs p, const SampleArgs q)
+__global__ void __launch_bounds__(Z::bound, 1) linep_sample_kernel(const LineArgs p, const SampleArgs q)
 {
     extern __shared__ float4 smp[];
     Z z;

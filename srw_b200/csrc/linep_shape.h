@@ -36,6 +36,7 @@ struct PShape {
     const int* t1;                    // offsets of the stages' twiddle tables (first, second transform)
     const int* t2;
     static constexpr bool fixed = false;
+    static constexpr int bound = 512; // (see FShape)
     SRWG_HD int tw1(int s) const { return t1[s]; }
     SRWG_HD int tw2(int s) const { return t2[s]; }
     SRWG_HD int N() const { return N_; }
@@ -77,6 +78,14 @@ template <int R0, int R1, int R2, int R3, int TT> struct FShape {
         return s == 0 ? R0 * R1 * R2 * R3 : s == 1 ? R1 * R2 * R3 : s == 2 ? R2 * R3 : s == 3 ? R3 : 1;
     }
     SRWG_HD static constexpr int pitch() { return L(1) | 1; }
+    // threads the kernels' registers are bounded for: 640 (96 registers) where that puts more CTAs on an SM,
+    // 512 (128 registers) where it only spills.  Warps per SM are 21 instead of 16: CTAs of a power of two
+    // threads gain nothing (two of 256 either way), others do (2240 x 1536, drifts: 239 to 216 us; quadratic
+    // drifts at 4096^2 would go from 935 to 1000), and so do short radix-8 lines (512: 32.7 to 30.8; 16 x 8 x 8
+    // at 1024 would go from 65 to 69, 8 x 8 x 4 at 256 on 32 threads from 43 to 47 for a batch of 8).
+    static constexpr bool pow2T = (TT & (TT - 1)) == 0;
+    static constexpr int maxR = R0 > R1 ? (R0 > R2 ? R0 : R2) : (R1 > R2 ? R1 : R2);
+    static constexpr int bound = TT < 64 ? 512 : !pow2T || maxR <= 8 ? 640 : 512;
     SRWG_HD static constexpr int divR(int u, int s) { return (int)((unsigned)u / (unsigned)R(s)); }
     SRWG_HD static constexpr int divL(int u, int s) { return (int)((unsigned)u / (unsigned)L(s)); }
     SRWG_HD static constexpr int divB(int u, int s)
