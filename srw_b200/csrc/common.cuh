@@ -183,72 +183,6 @@ template <int R, int DIR> __device__ __forceinline__ void dftR(float2* v, const 
     else dftg<R, DIR>(v, tw, N / R);
 }
 
-// One Stockham autosort stage on a line of N points in shared memory.  Thread t of T owns the
-// butterflies j = t, t+T, ...; all its inputs are read into registers before the barrier, so the
-// stage works in place.  Ns = product of the radices already applied.
-template <int R, int DIR>
-__device__ __forceinline__ void stockham_stage(float2* s, int N, int Ns, const float2* __restrict__ tw, int t, int T,
-                                               bool active)
-{
-    constexpr int MAXB = (16 + R - 1) / R;
-    const int NR = N / R;
-    const int tws = N / (Ns * R);
-    float2 v[MAXB][R];
-#pragma unroll
-    for (int b = 0; b < MAXB; b++) {
-        int j = t + b * T;
-        if (active && j < NR) {
-            int k = j % Ns;
-#pragma unroll
-            for (int r = 0; r < R; r++) {
-                float2 x = s[j + r * NR];
-                if (r > 0 && k != 0) {
-                    float2 w = __ldg(&tw[k * tws * r]);
-                    if (DIR < 0) w.y = -w.y;
-                    x = cmul(x, w);
-                }
-                v[b][r] = x;
-            }
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int b = 0; b < MAXB; b++) {
-        int j = t + b * T;
-        if (active && j < NR) {
-            dftR<R, DIR>(v[b], tw, N);
-            int k = j % Ns;
-            int base = (j / Ns) * Ns * R + k;
-#pragma unroll
-            for (int r = 0; r < R; r++) s[base + r * Ns] = v[b][r];
-        }
-    }
-    __syncthreads();
-}
-
-template <int DIR>
-__device__ void run_fft(float2* s, int N, const int* radix, int nst, const float2* __restrict__ tw, int t, int T,
-                        bool active)
-{
-    int Ns = 1;
-    for (int st = 0; st < nst; st++) {
-        int R = radix[st];
-        switch (R) {
-        case 16: stockham_stage<16, DIR>(s, N, Ns, tw, t, T, active); break;
-        case 8: stockham_stage<8, DIR>(s, N, Ns, tw, t, T, active); break;
-        case 4: stockham_stage<4, DIR>(s, N, Ns, tw, t, T, active); break;
-        case 2: stockham_stage<2, DIR>(s, N, Ns, tw, t, T, active); break;
-        case 3: stockham_stage<3, DIR>(s, N, Ns, tw, t, T, active); break;
-        case 5: stockham_stage<5, DIR>(s, N, Ns, tw, t, T, active); break;
-        case 7: stockham_stage<7, DIR>(s, N, Ns, tw, t, T, active); break;
-        case 11: stockham_stage<11, DIR>(s, N, Ns, tw, t, T, active); break;
-        case 13: stockham_stage<13, DIR>(s, N, Ns, tw, t, T, active); break;
-        default: break;
-        }
-        Ns *= R;
-    }
-}
-
 // ------------------------------------------------------------------------------------------------
 // point-wise operators
 // ------------------------------------------------------------------------------------------------
@@ -283,141 +217,7 @@ __device__ __forceinline__ void pw_eval(const PwOps& pw, int i, int j, double& p
     }
 }
 
-// W[k] = factor(k) * V[src(k)] for the chain: [post of a previous transform] -> [point-wise] ->
-// [mirror along the line] -> [pre of the next transform].
-struct Chain {
-    int rs1, sh1;
-    double a1;
-    float sc1;
-    const PwOps* pw;
-    int mir;
-    int rs2, sh2;
-    double a2;
-    int axis;
-};
-
-__device__ __forceinline__ float2 chain_eval(const Chain& c, int k, int N, int line, int& src)
-{
-    const int half = N >> 1;
-    double ph = 0.;
-    bool hasph = false, zero = false;
-    float sg = 1.f;
-    float2 f = make_float2(1.f, 0.f);
-    int m = k;
-    if (c.rs2) {                      // rotate then sign: W[k] = (-1)^k M[(k+N/2)%N]
-        m = k + half; if (m >= N) m -= N;
-        if (k & 1) sg = -sg;
-    }
-    if (c.sh2) { ph += c.a2 * (double)(m - half); hasph = true; }   // shift-before (on the source index)
-    int i = c.mir ? (N - 1 - m) : m;
-    if (c.pw) {
-        int ix = c.axis == 0 ? i : line, jz = c.axis == 0 ? line : i;
-        double p0 = ph;
-        pw_eval(*c.pw, ix, jz, ph, f, zero);
-        hasph = hasph || (ph != p0) || c.pw->has_quad || c.pw->has_ang;
-    }
-    int s = i;
-    if (c.rs1) {                      // sign then rotate: Z[i] = (-1)^s Y[s], s = (i+N/2)%N
-        s = i + half; if (s >= N) s -= N;
-        if (s & 1) sg = -sg;
-    }
-    if (c.sh1) { ph += c.a1 * (double)(i - half); hasph = true; }   // shift-after (on the output index)
-    src = s;
-    float sc = sg * c.sc1;
-    float2 r = make_float2(sc * f.x, sc * f.y);
-    if (hasph) r = cmul(r, expi(ph));
-    if (zero) r = make_float2(0.f, 0.f);
-    return r;
-}
-
-__device__ __forceinline__ bool chain_trivial(const Chain& c)
-{
-    return !c.rs1 && !c.sh1 && c.sc1 == 1.f && c.pw == nullptr && !c.mir && !c.rs2 && !c.sh2;
-}
-
-// register-staged in-place gather on one line: s[k] <- factor(k) s[src(k)]
-__device__ __forceinline__ void gather_pass(float2* s, int N, int line, const Chain& c, int t, int T, bool active)
-{
-    float2 tmp[16];
-#pragma unroll
-    for (int v = 0; v < 16; v++) {
-        int k = t + v * T;
-        if (active && k < N) {
-            int src;
-            float2 f = chain_eval(c, k, N, line, src);
-            tmp[v] = cmul(f, s[src]);
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int v = 0; v < 16; v++) {
-        int k = t + v * T;
-        if (active && k < N) s[k] = tmp[v];
-    }
-    __syncthreads();
-}
-
-// chain of a general (even) line length with its along-line factors in the plan's tables:
-// W[k] = tab[k] * extra(i(k), line) * V[src(k)], m = rot2(k), i = mirror(m), src = rot1(i)
-struct ChainG {
-    int rs1, mir, rs2;
-    int tab;                 // offset of the along-line factors in the plan's tables, or -1
-    int extra;               // the pass's non-separable work applies to this chain
-};
-
-__device__ __forceinline__ int chainG_src(const ChainG& c, int k, int N, int& i)
-{
-    const int h = N >> 1;
-    int m = k;
-    if (c.rs2) { m = k + h; if (m >= N) m -= N; }
-    i = c.mir ? (N - 1 - m) : m;
-    int s = i;
-    if (c.rs1) { s = i + h; if (s >= N) s -= N; }
-    return s;
-}
-
-__device__ __forceinline__ bool chainG_trivial(const ChainG& c)
-{
-    return !c.rs1 && !c.mir && !c.rs2 && c.tab < 0 && !c.extra;
-}
-
 __device__ __forceinline__ void extra_eval(const PwOps& e, int i, int j, float2& f, bool& zero, const float2* tabs);
-
-template <bool EXTRA = true>
-__device__ __forceinline__ float2 chainG_factor(const ChainG& c, int k, int i, int line, const float2* tabs,
-                                                const PwOps* ex, int axis)
-{
-    float2 f = c.tab >= 0 ? __ldg(&tabs[c.tab + k]) : make_float2(1.f, 0.f);
-    if (EXTRA && c.extra) {
-        bool zero = false;
-        extra_eval(*ex, axis == 0 ? i : line, axis == 0 ? line : i, f, zero, tabs);
-        if (zero) f = make_float2(0.f, 0.f);
-    }
-    return f;
-}
-
-// register-staged in-place gather on one line through a table chain: s[k] <- factor(k) s[src(k)]
-__device__ __forceinline__ void gather_pass_t(float2* s, int N, int line, const ChainG& c, int t, int T, bool active,
-                                              const float2* tabs, const PwOps* ex, int axis)
-{
-    float2 tmp[16];
-#pragma unroll
-    for (int v = 0; v < 16; v++) {
-        const int k = t + v * T;
-        if (active && k < N) {
-            int i;
-            const int src = chainG_src(c, k, N, i);
-            tmp[v] = cmul(chainG_factor(c, k, i, line, tabs, ex, axis), s[src]);
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int v = 0; v < 16; v++) {
-        const int k = t + v * T;
-        if (active && k < N) s[k] = tmp[v];
-    }
-    __syncthreads();
-}
 
 // RadPointModifier_PropToWaistBeyondParax (sroptdrf.h:712-754): exp(i k L (sqrt(1 + X) - 1)), or with
 // k L sqrt(1 + X) on the path-length option, X = -lambda^2 (qx^2 + qz^2); the square root for

@@ -1,9 +1,6 @@
-// General FFT lengths with a specialised line-pass kernel (linen.cuh): 2^a m, a >= 4, for the odd parts
-// m that range / resolution factors of 1.25, 1.5, 1.75 and their products give on 256 .. 1024-point
-// inputs (3, 5, 7, 9, 15, 25, 35), from 320 to 7168 points.  Each is compiled as its own unit
-// (linen.cu with SRWG_LINEN=N); other general lengths run the run-time-scheduled pass (lineg.cuh).
-// The powers of two are compiled as well: the autotuner chooses, per axis and length, between them
-// and the power-of-two pass (line2.cuh).
+// The general lengths (2^a m, a >= 4) that range / resolution factors of 1.25, 1.5, 1.75 and their products
+// give on 256 .. 1024-point inputs, from 320 to 7168 points: the autotuner measures lines per CTA for these
+// and the powers of two (their schedules: linep_lengths.h).
 #pragma once
 
 #define SRWG_LINEN_LENGTHS(X)                                                                            \
