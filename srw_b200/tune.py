@@ -1,11 +1,10 @@
 """Autotuner of the FFT line passes' launch shapes (the reference has none: FFTW plans per call,
 gmfft.cpp:295; its CUDA build caches cuFFT plans, gmfft.h:182-187).
 
-For every line length with a compile-time kernel (powers of two and the general lengths of
-csrc/linen_lengths.h) it times the two passes of an N x N propagation to the waist (a row pass and
-a column pass, the headline beamline's FFT) for every valid kernel family (powers of two: the
-power-of-two pass or the specialised pass) and number of lines per CTA of each pass -- which is
-also the CTA size and, for the column pass, the width of the column blocks the row pass writes --
+For every tuned line length (powers of two and the general lengths of csrc/linen_lengths.h) it times the two passes of an N x N propagation to the waist (a row pass and
+a column pass, the headline beamline's FFT) for every valid number of lines per CTA of each pass (two
+lines make a pair; the kernel family is kept in the table and chooses nothing) -- which is also the CTA
+size and, for the column pass, the width of the column blocks the row pass writes --
 with CUDA events on the launching stream and L2 flushed between repetitions, keeps the fastest
 pair and writes
 
