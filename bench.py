@@ -50,14 +50,12 @@ SIG_E = 1e-3                                   # relative electron energy spread
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch of a pass, from an ncu
 # capture of this workload (the plain passes' summary under profiles/); keyed by the pass tuple of
 # Plan.kernels().  Re-captured whenever the kernel changes.
-TRAFFIC = {('line_cols', 4096, 4096): 37369856 + 216899840,
-           ('line_rows', 4096, 4096): 5258752 + 2144256,
-           ('resize', 1024, 1024, 4096, 4096): 1373696 + 512}
-# the same per electron of the batched passes at the learned factors (ncu on a batch of 8, the
-# learned batch's summary under profiles/); a launch moves this times its electrons
-TRAFFIC_PER_ELECTRON = {('line_cols', 1536, 1600): (69851904 + 29201664) // 8,
-                        ('line_rows', 1536, 1600): (19814912 + 20619776) // 8,
-                        ('resize', 1024, 1024, 1536, 1600): (2238208 + 202240) // 8}
+# (Not captured for the plain passes of the present kernels.)
+TRAFFIC = {}
+# the same per electron of the batched passes at the learned factors (ncu on a batch of 8); a launch
+# moves this times its electrons
+TRAFFIC_PER_ELECTRON = {('line_cols', 1536, 1600): (19659008 + 3882752) // 8,
+                        ('line_rows', 1536, 1600): (35271680 + 67584) // 8}
 
 
 # ------------------------------------------------------------------------------------------------
@@ -379,6 +377,11 @@ def batched_passes(me, offs, stream, peak, peak_src, where):
     if inten:
         k = ks[-1]
         alg[-1] = 2 * 8 * k[1] * k[2] + 4 * k[1] * k[2]
+        if k[0] == 'line_rows' and 2 * getattr(me, 'ny', k[2]) < k[2]:
+            # only rows around the detector's are read, and their sums are written: what is counted is the
+            # captured traffic where there is one, else two rows per detector row
+            t = TRAFFIC_PER_ELECTRON.get(tuple(k))
+            alg[-1] = t if t is not None else 2 * 8 * k[1] * 2 * me.ny
     kd = int(np.argmax(per))
     achieved = alg[kd] * nb / (per[kd] / 1000.) / 1e9
     return {"bound": "hbm", "kernel": "%s %s (batch of %d)" % (ks[kd][0], 'x'.join(map(str, ks[kd][1:])), nb),
