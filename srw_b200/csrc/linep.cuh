@@ -917,7 +917,7 @@ __global__ void __launch_bounds__(Z::bound, 1) linep_kernel(const LineArgs p)
     x.sg0 = x.sg1 = nullptr;
     __shared__ uint64_t bar;
     pdl_wait();
-    if (p.bulk && d.zwin && d.za0 <= d.za1) {
+    if (p.bulk && d.zwin && d.blk_in == p.L && d.za0 <= d.za1) {
         // the tile is one block of lines: its nonzero points lie together and arrive in shared memory,
         // behind the slots, by one bulk copy per component while the chains are set up
         float2* stg = reinterpret_cast<float2*>(smp + Lp * p.P);

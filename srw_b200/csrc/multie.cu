@@ -473,9 +473,11 @@ static int flush(srwgMultiE& m, int nb, std::vector<KernelDesc>& ks, cudaStream_
     MTRY(cudaStreamWaitEvent(st, m.staged[s], 0));
     int r = 0;
     if (m.useGraph && nb == m.maxBatch && m.tev.empty()) {
-        // the graph holds the launch shapes; a batch whose resize tiles are larger needs a new one
-        // (and launches only the windows' CTAs: a batch whose windows reach beyond them too)
-        bool fits = m.graph[s] != nullptr && m.graphKs[s].size() == ks.size();
+        // the graph holds the kernels and launch shapes of its passes; a batch of another structure
+        // (kinds of passes, blocks, sampled rows) needs a new one, and so does one whose resize tiles are
+        // larger (it launches only the windows' CTAs: one whose windows reach beyond them too)
+        const bool had = m.graph[s] != nullptr && same_structure(m.graphKs[s], ks);
+        bool fits = had;
         for (size_t i = 0; fits && i < ks.size(); i++) {
             const KernelDesc &a = ks[i], &g = m.graphKs[s][i];
             if (a.kind == K_RESIZE &&
@@ -485,11 +487,10 @@ static int flush(srwgMultiE& m, int nb, std::vector<KernelDesc>& ks, cudaStream_
             if (a.kind == K_LINE && a.line.zwin && a.line.zl1 > g.line.zl1) fits = false;
         }
         if (!fits) {
-            // the new graph's shapes cover this batch, the graph it replaces and a little more (tiles of
+            // the new graph's shapes cover this batch, one of its structure it replaces and a little more (tiles of
             // the resize, a line block or two of window), so that batches seldom need another one: an
             // instantiation costs milliseconds of host time
             std::vector<KernelDesc> cap = ks;
-            const bool had = m.graph[s] && m.graphKs[s].size() == cap.size();
             for (size_t i = 0; i < cap.size(); i++) {
                 if (cap[i].kind == K_RESIZE) {
                     ResizeDesc& r = cap[i].rs;

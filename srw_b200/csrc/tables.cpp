@@ -237,7 +237,7 @@ static void quartic_tables(std::vector<float2>& T, LineDesc& d, int N, int nl)
     d.has_extra = 0;
     if (ph < 0x1p-27) {
         T.resize(before);
-        d.ang = 0;
+        d.ang = d.qtab = d.qline = 0;
     } else {
         d.ang = ph < 0.03 ? 1 : 2;
     }

@@ -1,0 +1,50 @@
+"""Multi-electron runs whose detector rows lie about twice as far apart as the output's rows: the rule of
+the sampled last pass (two output rows or more per detector row) then depends on the photon energy of each
+electron.  The mean against the FP64 oracle run electron by electron, with replayed graphs and without;
+its bar as in test_sampled_rows.py (FP32 transforms accurate to about 5e-7: 1e-5 leaves a factor of
+ten)."""
+import numpy as np
+import pytest
+
+from srw_b200.multie import sample_offsets
+from tests.helpers import C1, PP, O, beamline, gaussian, make_wfr, rel_l2
+from tests.test_multie import SIG, oracle_sum
+
+torch = pytest.importorskip('torch')
+SC = dict(Rx=20., Ry=20., dRx=0.2, dRy=0.2, xc=0., yc=0.)
+
+
+def half_rows_case(n=12):
+    """128 x 512 to 320 x 1280, a detector of half the rows over the same range (2.0016 output rows apart),
+    electrons two by two on either side of the rule."""
+    ex, _, mesh = gaussian(128, E=2012., sig=0.35e-3, r=1.5e-3, R=20., ny=512)
+    ey = (0.3 + 0.2j) * ex
+    pp = [PP(), PP(0, 1.25, 2., 1.25, 2.), PP(4)]
+    o = O.Wfr.from_srwl(ex, ey, mesh, 20., 20., 0.2, 0.2, 0., 0.)
+    O.propagate(o, [tuple(e) for e in C1], pp)
+    m = o.out_mesh()
+    assert (m['nx'], m['ny']) == (320, 1280)
+    acc = dict(nx=96, ny=640, eStart=mesh['eStart'], **{k: m[k] for k in ('xStart', 'xFin', 'yStart', 'yFin')})
+    offs = sample_offsets(n, *SIG, seed=5, sig_e=1e-3)
+    offs[:, 4] = np.where(np.arange(n) // 2 % 2 == 0, -1e-3, 1e-3)
+    return ex, ey, mesh, pp, acc, offs
+
+
+def need_gpu():
+    if not torch.cuda.is_available():
+        pytest.skip('no CUDA device')
+
+
+@pytest.mark.gpu
+def test_graphs_of_mixed_electrons_vs_oracle():
+    need_gpu()
+    from srw_b200.multie import MultiE
+    ex, ey, mesh, pp, acc, offs = half_rows_case()
+    want = oracle_sum(dict(ex=ex, ey=ey, mesh=mesh), SC, C1, pp, acc, offs) / len(offs)
+    assert np.abs(want).max() > 0
+    w = make_wfr(ex, ey, mesh, **SC)
+    for graph, batch in ((False, 4), (True, 1), (True, 2), (True, 4)):
+        me = MultiE(w, beamline(C1, pp), acc, max_batch=batch, graph=graph)
+        me.add(offs)
+        assert me.count() == len(offs)
+        assert rel_l2(me.mean(), want) < 1e-5, (graph, batch)
