@@ -124,6 +124,13 @@ __global__ void __launch_bounds__(256) accum_parts_kernel(const double* __restri
     acc[i] += s;
 }
 
+// Whether a run's last pass transforms only the rows its detector samples: where a detector row (azStep
+// apart) lies two output rows (zStep) or more from the next; closer ones would transform rows twice (all rows
+// then, once).  Decided once per run, from the base wavefront: each electron's own step follows its photon
+// energy, and electrons on either side of the rule would not share a batch.  (Either form is right at any
+// ratio.)
+static bool sampled_rows(double azStep, double zStep) { return azStep >= 2. * std::fabs(zStep); }
+
 // magnitude^2 of the n complex values at float2 offset `off` of the plan's tables when all of them
 // have it (relative spread within 1e-6), else -1
 static double flat_mag2(const std::vector<float2>& T, long long off, int n)
@@ -144,12 +151,10 @@ static double flat_mag2(const std::vector<float2>& T, long long off, int n)
 // sample instead of two complex values).  Where its output factors -- the output chain's table along
 // the lines and every chain's line factor -- have one magnitude, |f v|^2 = |f|^2 |v|^2: the pass
 // skips them and scales the intensity by that magnitude squared.
-// Along the rows, where a detector row (azStep apart, anx columns) lies two output rows (zStep) or more
-// from the next, only the two rows around each are transformed, in one pass with the accumulation
-// (out_int 2): 2 zStep / azStep of the rows, and no intensities written and read back.  Closer detector rows would
-// transform rows twice: all rows then, once (out_int 1).
-static void mark_intensity_pass(std::vector<KernelDesc>& ks, const std::vector<float2>& tables, int anx, double azStep,
-                                double zStep)
+// Along the rows of a run with sampled rows (sampled_rows), only the two rows around each detector row (anx
+// columns) are transformed, in one pass with the accumulation (out_int 2): 2 zStep / azStep of the rows, and
+// no intensities written and read back.
+static void mark_intensity_pass(std::vector<KernelDesc>& ks, const std::vector<float2>& tables, int anx, bool sampled)
 {
     for (size_t i = ks.size(); i-- > 0;) {
         if (reads_only(ks[i].kind)) continue;
@@ -163,7 +168,7 @@ static void mark_intensity_pass(std::vector<KernelDesc>& ks, const std::vector<f
                 if (d.axis == 1 && d.blk_out == 0) d.blk_out = pair_block(N, d.nx);
                 LineLaunch shape;
                 memset(&shape, 0, sizeof(shape));
-                if (d.axis == 0 && azStep >= 2. * std::fabs(zStep) && line_config(d, shape) == 0 && sample_fits(shape, anx)) {
+                if (d.axis == 0 && sampled && line_config(d, shape) == 0 && sample_fits(shape, anx)) {
                     d.out_int = 2;
                     // single rows are read, not blocks of them: row-major before this pass
                     if (d.blk_in > 0 && i > 0 && ks[i - 1].kind == K_LINE) {
@@ -216,6 +221,7 @@ struct srwgMultiE {
     // common mesh and FP64 accumulator
     int anx = 0, anz = 0;
     double axStart = 0, axStep = 0, azStart = 0, azStep = 0;
+    bool sampled = false;                // the last pass transforms only the rows the detector samples
     double* dAcc = nullptr;
     double* dSnap = nullptr;             // the accumulator as it was before the current add call
     bool ownAcc = true;                  // false: caller-provided accumulator (srwgMultiESetAccumulator)
@@ -594,7 +600,10 @@ extern "C" SRWG_API int srwgMultiECreate(const SRWLWfr* pBase, const SRWLOptC* p
     pl.numMoments = false;               // only the intensity is kept: no moment passes
     pl.inPhase = true;                   // the electrons' kick (here zero): the same passes as theirs
     r = pl.plan(pBase, pOpt);
-    if (!r) mark_intensity_pass(pl.kernels, pl.tables, m->anx, m->azStep, pl.w.zStep);
+    if (!r) {
+        m->sampled = sampled_rows(m->azStep, pl.w.zStep);
+        mark_intensity_pass(pl.kernels, pl.tables, m->anx, m->sampled);
+    }
     if (r) { set_last_detail(pl.err); delete m; return r; }
     m->nIn = (size_t)m->nx * m->nz;
     m->nOut = (size_t)pl.w.nx * pl.w.nz;
@@ -806,7 +815,7 @@ static int add_body(srwgMultiE* m, int n, const double* arOffsets, int stride, c
                     pls[k].inKz = eps[k].kz;
                     pls[k].inC = -(eps[k].kx * eps[k].dx + eps[k].kz * eps[k].dz);
                     rcs[k] = pls[k].plan(&w, m->opt);
-                    if (!rcs[k]) mark_intensity_pass(pls[k].kernels, pls[k].tables, m->anx, m->azStep, pls[k].w.zStep);
+                    if (!rcs[k]) mark_intensity_pass(pls[k].kernels, pls[k].tables, m->anx, m->sampled);
                 }
             };
             m->pool->run(std::min(nthr, cnt), work);
@@ -879,7 +888,7 @@ extern "C" SRWG_API int srwgMultiEInfo(srwgMultiE* m, int* nPasses, int* intensi
     pl.inPhase = true;
     int r = pl.plan(&m->base, m->opt);
     if (r) { set_last_detail(pl.err); return r; }
-    mark_intensity_pass(pl.kernels, pl.tables, m->anx, m->azStep, pl.w.zStep);
+    mark_intensity_pass(pl.kernels, pl.tables, m->anx, m->sampled);
     if (nPasses) *nPasses = (int)pl.kernels.size();
     if (intensityPass) *intensityPass = intensity_pass(pl.kernels) ? 1 : 0;
     if (desc && descLen > 0) {

@@ -48,3 +48,14 @@ def test_graphs_of_mixed_electrons_vs_oracle():
         me.add(offs)
         assert me.count() == len(offs)
         assert rel_l2(me.mean(), want) < 1e-5, (graph, batch)
+
+
+@pytest.mark.gpu
+def test_mixed_electrons_run_as_one_batch():
+    """A timed add refuses electrons that do not run as one batch."""
+    need_gpu()
+    from srw_b200.multie import MultiE
+    ex, ey, mesh, pp, acc, offs = half_rows_case()
+    me = MultiE(make_wfr(ex, ey, mesh, **SC), beamline(C1, pp), acc, max_batch=len(offs), graph=False)
+    me.add_timed(offs)
+    assert me.count() == len(offs)
