@@ -222,6 +222,7 @@ struct srwgMultiE {
     int anx = 0, anz = 0;
     double axStart = 0, axStep = 0, azStart = 0, azStep = 0;
     bool sampled = false;                // the last pass transforms only the rows the detector samples
+    std::vector<int> ang;                // class of each pass's quartic phase (base wavefront)
     double* dAcc = nullptr;
     double* dSnap = nullptr;             // the accumulator as it was before the current add call
     bool ownAcc = true;                  // false: caller-provided accumulator (srwgMultiESetAccumulator)
@@ -602,6 +603,7 @@ extern "C" SRWG_API int srwgMultiECreate(const SRWLWfr* pBase, const SRWLOptC* p
     r = pl.plan(pBase, pOpt);
     if (!r) {
         m->sampled = sampled_rows(m->azStep, pl.w.zStep);
+        for (const KernelDesc& k : pl.kernels) m->ang.push_back(k.kind == K_LINE ? k.line.ang : 0);
         mark_intensity_pass(pl.kernels, pl.tables, m->anx, m->sampled);
     }
     if (r) { set_last_detail(pl.err); delete m; return r; }
@@ -609,7 +611,11 @@ extern "C" SRWG_API int srwgMultiECreate(const SRWLWfr* pBase, const SRWLOptC* p
     m->nOut = (size_t)pl.w.nx * pl.w.nz;
     m->perWork = (size_t)std::max<long long>(pl.maxElems, 2);
     m->perWork += m->perWork & 1;        // 16-byte aligned fields
-    const size_t tabBytes = ((pl.tables.size() * sizeof(float2) + 255) & ~(size_t)255) + 4096;   // slack for alignment pads
+    // room for alignment pads, and for the quartic phase's tables where the base wavefront needs none
+    size_t slack = 4096;
+    for (const KernelDesc& k : pl.kernels)
+        if (k.kind == K_LINE && k.line.f1 && k.line.f2) slack += (size_t)(k.line.nx + k.line.nz + 2) * sizeof(float);
+    const size_t tabBytes = ((pl.tables.size() * sizeof(float2) + slack + 255) & ~(size_t)255);
     m->descOff = tabBytes;
     m->constStride = (tabBytes + pl.kernels.size() * sizeof(KernelDesc) + 255) & ~(size_t)255;
 #define MALLOC(p, n)                                                                 \
@@ -811,6 +817,7 @@ static int add_body(srwgMultiE* m, int n, const double* arOffsets, int stride, c
                     pls[k].numMoments = false;
                     // the kick kx (x - dx) + kz (z - dz) on the electron's (shifted) mesh
                     pls[k].inPhase = true;
+                    pls[k].likeAng = &m->ang;
                     pls[k].inKx = eps[k].kx;
                     pls[k].inKz = eps[k].kz;
                     pls[k].inC = -(eps[k].kx * eps[k].dx + eps[k].kz * eps[k].dz);

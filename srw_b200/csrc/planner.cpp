@@ -1798,7 +1798,7 @@ int Planner::finalize()
             return SRWG_ERR_UNSUPPORTED;
         }
     }
-    build_tables(kernels, tables);
+    build_tables(kernels, tables, likeAng);
     // transmission tables after the separable ones (each double of a (T, OPD) pair in one float2
     // slot), and their offsets into every point-wise description that uses them
     if (!trTables_.empty()) {

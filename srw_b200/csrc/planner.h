@@ -83,8 +83,9 @@ void fill_moment_desc(const WfrState& w, MomDesc& d, MomOp& op);
 void single_moment_pass(const WfrState& w, KernelDesc& k, MomOp& op, std::vector<float2>& tables);
 void moments_from_sums(const double* S, const MomOp& op, double* momX, double* momZ);
 
-// fills the separable point-wise tables of every pass (tables.cpp)
-void build_tables(std::vector<KernelDesc>& ks, std::vector<float2>& tables);
+// fills the separable point-wise tables of every pass (tables.cpp); like: the class of each pass's quartic phase
+// in the plan whose batches these passes join (LineRun::ang)
+void build_tables(std::vector<KernelDesc>& ks, std::vector<float2>& tables, const std::vector<int>* like = nullptr);
 
 // an intensity extraction after an element (srwlPropagElecField's arID / arIM / arI lists): after
 // element `elem` (0-based; the number of elements: after the post-resize), request `index`
@@ -134,6 +135,8 @@ public:
     // field before the first element, fused into the first pass (the angular kick of a macro-electron)
     bool inPhase = false;
     double inKx = 0, inKz = 0, inC = 0;
+    // the quartic phases' classes of the plan whose batches this one's passes join, one per pass (see build_tables)
+    const std::vector<int>* likeAng = nullptr;
     int nStages = 0;                     // stage boundaries passed
     WfrState stageIn;                    // mesh of the current stage's input
 

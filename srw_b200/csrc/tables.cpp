@@ -201,11 +201,25 @@ static ChainTab chain_table(std::vector<float2>& T, int N, int nLine, int rs1, i
     return ct;
 }
 
+// The class of a quartic phase of at most ph rad: 0 below 2^-27 rad (a quarter of an FP32 rounding of the factor),
+// left out; 1 below 0.03 rad, by its series; 2 any.  `like` >= 0: the class of the wavefront this one runs in a
+// batch with (the base of a multi-electron run), kept within a quarter beyond its limits, since a batch runs one
+// class and the photon energies of its electrons differ by some 1e-3.  (A quarter beyond, the phase left out is
+// a third of a rounding and the series' next term 6e-10.)
+static int quartic_class(double ph, int like)
+{
+    const double lim[2] = {0x1p-27, 0.03};
+    if (like == 0 && ph < 1.25 * lim[0]) return 0;
+    if (like == 1 && ph >= lim[0] / 1.25 && ph < 1.25 * lim[1]) return 1;
+    if (like == 2 && ph >= lim[1] / 1.25) return 2;
+    return ph < lim[0] ? 0 : ph < lim[1] ? 1 : 2;
+}
+
 // The quartic part of the angular transfer function (phase c0 q2 (c1 q2)(1 + 2 c1 q2), q2 = qx^2 + qz^2) as
 // the only non-separable work of a pass with two transforms: FP32 tables of qx^2 and qz^2 (from FP64)
-// along the line and per line instead of the point-by-point evaluation.  Where it is below 2^-27 rad
-// everywhere (a quarter of an FP32 rounding of the factor) it is dropped.
-static void quartic_tables(std::vector<float2>& T, LineDesc& d, int N, int nl)
+// along the line and per line instead of the point-by-point evaluation, or nothing where it is below any
+// effect (quartic_class).
+static void quartic_tables(std::vector<float2>& T, LineDesc& d, int N, int nl, int like)
 {
     PwOps& e = d.extra;
     if (!e.has_ang || e.has_bpx || e.has_tr || e.nmask) return;
@@ -235,11 +249,10 @@ static void quartic_tables(std::vector<float2>& T, LineDesc& d, int N, int nl)
     d.qc1 = (float)e.c1;
     const double q2 = ma + ml, c1q2 = std::fabs(e.c1 * q2), ph = std::fabs(e.c0 * q2) * c1q2 * (1. + 2. * c1q2);
     d.has_extra = 0;
-    if (ph < 0x1p-27) {
+    d.ang = quartic_class(ph, like);
+    if (d.ang == 0) {
         T.resize(before);
-        d.ang = d.qtab = d.qline = 0;
-    } else {
-        d.ang = ph < 0.03 ? 1 : 2;
+        d.qtab = d.qline = 0;
     }
 }
 
@@ -308,7 +321,7 @@ static int tile_extent(const std::vector<float2>& T, long long off, int nNew, lo
     return best;
 }
 
-void build_tables(std::vector<KernelDesc>& ks, std::vector<float2>& T)
+void build_tables(std::vector<KernelDesc>& ks, std::vector<float2>& T, const std::vector<int>* like)
 {
     T.clear();
     // room for the largest tables the passes can ask for (no reallocation while they are added)
@@ -355,7 +368,8 @@ void build_tables(std::vector<KernelDesc>& ks, std::vector<float2>& T)
             if (d.f2) { rs2 = d.f2_pre.rs; sh2 = d.f2_pre.has_shift; a2 = d.f2_pre.shift_a; }
             d.t_mid = chain_table(T, N, nl, rs1, sh1, a1, sc1, pA, pL, scale, d.mirror_along, rs2, sh2, a2);
             d.ang = 0;
-            if (d.has_extra && d.f1 && d.f2 && pair_supported(N)) quartic_tables(T, d, N, nl);
+            if (d.has_extra && d.f1 && d.f2 && pair_supported(N))
+                quartic_tables(T, d, N, nl, like && like->size() == ks.size() ? (*like)[&k - ks.data()] : -1);
             d.t_fin.tab = d.t_fin.ltab = -1;
             if (d.f2)
                 d.t_fin = chain_table(T, N, nl, d.f2_post.rs, d.f2_post.has_shift, d.f2_post.shift_a, d.f2_post.scale,

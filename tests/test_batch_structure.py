@@ -59,3 +59,26 @@ def test_mixed_electrons_run_as_one_batch():
     me = MultiE(make_wfr(ex, ey, mesh, **SC), beamline(C1, pp), acc, max_batch=len(offs), graph=False)
     me.add_timed(offs)
     assert me.count() == len(offs)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('E,r,L,sx', [(806.7, 8e-3, 10., 30e-6), (440.4, 5e-5, 1e-2, 1e-6)])
+def test_quartic_phase_at_its_limits(E, r, L, sx):
+    """Angular drifts whose largest quartic phase, pi lam L q2 (lam^2 q2 / 4), lies at 2^-27 rad (below: left
+    out) or 0.03 rad (below: by its series) and moves across with each electron's photon energy: one
+    batch, to the same mean.  (The factor's error on either side is below its FP32 rounding.)"""
+    need_gpu()
+    from srw_b200.multie import MultiE
+    ex, _, mesh = gaussian(512, E=E, sig=0.1 * r, r=r)
+    ey = (0.3 + 0.2j) * ex
+    sc = dict(Rx=0., Ry=0., dRx=0., dRy=0., xc=0., yc=0.)
+    el, pp = [('drift', L, 0), ('lens', 1e3, 1e3, 0., 0.), ('drift', L, 0)], [PP()] * 3
+    acc = dict(nx=64, ny=48, eStart=E, xStart=-0.8 * r, xFin=0.8 * r, yStart=-0.8 * r, yFin=0.8 * r)
+    offs = sample_offsets(6, sx, 1e-6, sx, 1e-6, seed=5, sig_e=1e-3)
+    offs[:, 4] = np.where(np.arange(6) % 2 == 0, 1e-3, -1e-3)
+    want = oracle_sum(dict(ex=ex, ey=ey, mesh=mesh), sc, el, pp, acc, offs) / len(offs)
+    assert np.abs(want).max() > 0
+    me = MultiE(make_wfr(ex, ey, mesh, **sc), beamline(el, pp), acc, max_batch=len(offs), graph=False)
+    me.add_timed(offs)
+    assert me.count() == len(offs)
+    assert rel_l2(me.mean(), want) < 1e-5
