@@ -343,23 +343,35 @@ static bool same_structure(const std::vector<KernelDesc>& a, const std::vector<K
     return true;
 }
 
+// captured launches name the buffers of their capture
+static void drop_graphs(srwgMultiE& m)
+{
+    for (int i = 0; i < 2; i++) {
+        if (m.graph[i]) cudaGraphExecDestroy(m.graph[i]);
+        m.graph[i] = nullptr;
+        m.graphKs[i].clear();
+    }
+}
+
 // device memory for what the last pass writes and the sampled pass's sums (made before a capture: every
-// launch sequence runs once directly first)
+// launch sequence runs once directly first); each buffer by itself, so that a call after one that found no
+// memory makes the missing ones
 static int ensure_out(srwgMultiE& m, int inten)
 {
     const size_t need = inten == 2 ? 0 : (size_t)m.sub * m.nOut * (inten ? sizeof(float) : 2 * sizeof(float2));
     if (need > m.outBytes) {
+        drop_graphs(m);
         cudaFree(m.dOut);
         m.dOut = nullptr;
         m.outBytes = 0;
         MTRY(cudaMalloc(&m.dOut, need));
         m.outBytes = need;
     }
-    if (inten == 2 && m.dPart == nullptr) {
+    if (inten == 2) {
         // about 1500 CTAs of one detector row each
         m.parts = std::min(m.sub, 1500 / m.anz + 1);
-        MTRY(cudaMalloc(&m.dPart, (size_t)m.parts * m.anx * m.anz * sizeof(double)));
-        MTRY(cudaMalloc(&m.dMask, (size_t)m.sub * 256 * sizeof(unsigned)));
+        if (m.dPart == nullptr) MTRY(cudaMalloc(&m.dPart, (size_t)m.parts * m.anx * m.anz * sizeof(double)));
+        if (m.dMask == nullptr) MTRY(cudaMalloc(&m.dMask, (size_t)m.sub * 256 * sizeof(unsigned)));
     }
     return 0;
 }
@@ -940,12 +952,7 @@ extern "C" SRWG_API int srwgMultiESetAccumulator(srwgMultiE* m, double* dAcc)
     cudaFree(m->dAcc);
     m->dAcc = dAcc;
     m->ownAcc = false;
-    for (int i = 0; i < 2; i++)              // captured launches name the old accumulator
-        if (m->graph[i]) {
-            cudaGraphExecDestroy(m->graph[i]);
-            m->graph[i] = nullptr;
-            m->graphKs[i].clear();
-        }
+    drop_graphs(*m);
     return 0;
 }
 
