@@ -82,3 +82,38 @@ def test_quartic_phase_at_its_limits(E, r, L, sx):
     me.add_timed(offs)
     assert me.count() == len(offs)
     assert rel_l2(me.mean(), want) < 1e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('rows,n,graph', [(200, 66, False), (200, 40, False), (200, 66, True), (1600, 40, False),
+                                          (1600, 66, True)])
+def test_batches_in_parts_equal_whole_batches(rows, n, graph):
+    """A batch whose work buffers would pass 8 GiB runs in parts (up to 66 electrons at 2048^2: 33 and 33, 40 of
+    them 33 and 7), with sampled rows and with all of them: the same electrons in batches of 8 give the
+    same sums up to the order of their FP64 additions (66 terms: 66 x 1.1e-16, a factor of ten left)."""
+    need_gpu()
+    from srw_b200.multie import MultiE
+    from srw_b200.plan import Plan
+    ex, _, mesh = gaussian(512, E=2012., sig=0.35e-3, r=1.5e-3, R=20.)
+    ey = (0.3 + 0.2j) * ex
+    pp = [PP(), PP(0, 2., 2., 2., 2.), PP(4)]
+    w = make_wfr(ex, ey, mesh, **SC)
+    m = Plan(w, beamline(C1, pp)).output_mesh()
+    assert (m['nx'], m['ny']) == (2048, 2048)
+    acc = dict(nx=100, ny=rows, eStart=mesh['eStart'], **{k: m[k] for k in ('xStart', 'xFin', 'yStart', 'yFin')})
+    offs = sample_offsets(n, *SIG, seed=8, sig_e=1e-3)
+    whole = MultiE(w, beamline(C1, pp), acc, max_batch=8, graph=False)
+    whole.add(offs)
+    want = whole.mean()
+    del whole
+    assert want.max() > 0
+    parts = MultiE(w, beamline(C1, pp), acc, max_batch=66, graph=graph)
+    for rep in range(4 if graph else 1):                         # both slots' graphs are captured, then replayed
+        parts.reset()
+        parts.add(offs)
+        assert parts.count() == n
+        np.testing.assert_allclose(parts.mean(), want, rtol=1e-13, atol=1e-13 * want.max())
+    if not graph:
+        parts.reset()
+        assert all(v > 0 for v in parts.add_timed(offs))
+        np.testing.assert_allclose(parts.mean(), want, rtol=1e-13, atol=1e-13 * want.max())
