@@ -4,8 +4,8 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <new>
-#include <system_error>
 #include <thread>
 
 namespace srwg {
@@ -162,8 +162,8 @@ cudaError_t copy_segments(HostRing& ring, int dev, const CopySeg* segs, int n, b
     int made = 0;
     try {
         for (; made < nt - 1; made++) th[made] = std::thread([&job, made]() { job.work(made + 1); });
-    } catch (const std::system_error&) {
-        // the threads that did start, and this one, take all blocks
+    } catch (const std::exception&) {
+        // no thread or no memory for one: the threads that did start, and this one, take all blocks
     }
     job.work(0);
     for (int i = 0; i < made; i++) th[i].join();
