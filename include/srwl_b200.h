@@ -296,7 +296,7 @@ SRWG_API int srwgWfrFeatures(const float* dEx, const float* dEy, int nx, int ny,
  * this runs the propagation of srwgPlanCreate + srwgPlanExecute without allocating any device
  * memory: the caller passes the input fields (dExIn/dEyIn, read only) and the output fields
  * (dExOut/dEyOut, outCapacity complex points each, device memory), and all intermediate data
- * lives in one fixed device array inside the library (11 MiB, held by every GPU that loads the
+ * lives in one fixed device array inside the library (12 MiB, held by every GPU that loads the
  * library until the process exits).  Limits: intermediate grids of at most 512 x 512 points,
  * 1 MiB of plan tables and 2 MiB of moment-pass results and scratch; larger propagations return
  * error 23904 (text: srwlUtiGetErrText).  Runs on the current device and `stream`; pWfrOut

@@ -11,9 +11,9 @@
 //
 // Limits: the largest intermediate grid of the planned passes may hold at most
 // SRWG_STATIC_WORK_POINTS complex points (512 x 512), and the plan's constant data at most
-// SRWG_STATIC_CONST_POINTS float2 (1 MiB), and the moment passes (result slots and scratch) at
-// most SRWG_STATIC_MOM_DOUBLES doubles (2 MiB); larger propagations are rejected with
-// SRWG_ERR_STATIC_LIMIT and a message giving the sizes.
+// SRWG_STATIC_CONST_POINTS float2 (1 MiB; counted as const_points does), and the moment passes (result
+// slots and scratch) at most SRWG_STATIC_MOM_DOUBLES doubles (2 MiB); larger propagations are rejected
+// with SRWG_ERR_STATIC_LIMIT and a message giving the sizes.
 //
 // Where the propagation recomputes the statistical moments from the field (an aperture that clips
 // the beam, an obstacle) and pWfrOut has moment arrays, the call waits for the stream to finish
@@ -41,6 +41,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -53,11 +54,12 @@
 #define SRWG_STATIC_WORK_POINTS (512 * 512)
 #define SRWG_STATIC_CONST_POINTS (128 * 1024)
 #define SRWG_STATIC_MOM_DOUBLES (256 * 1024)
-#define SRWG_STATIC_POINTS (4 * SRWG_STATIC_WORK_POINTS + SRWG_STATIC_CONST_POINTS + SRWG_STATIC_MOM_DOUBLES)
+#define SRWG_STATIC_CONST_ROOM (2 * SRWG_STATIC_CONST_POINTS)
+#define SRWG_STATIC_POINTS (4 * SRWG_STATIC_WORK_POINTS + SRWG_STATIC_CONST_ROOM + SRWG_STATIC_MOM_DOUBLES)
 
 namespace srwg {
 
-// [ work buffer A: Ex, Ey | work buffer B: Ex, Ey | constant data | moment slots and scratch ]  (11 MiB)
+// [ work buffer A: Ex, Ey | work buffer B: Ex, Ey | constant data | moment slots and scratch ]  (12 MiB)
 static __device__ __align__(256) float2 g_static_scratch[SRWG_STATIC_POINTS];
 
 static std::mutex g_static_mutex;
@@ -76,6 +78,30 @@ static int static_scratch(int dev, float2** out)
     g_static_addr[dev] = p;
     *out = p;
     return 0;
+}
+
+// The size that the limit on constant data is about: the passes' factors, a twiddle factor per point of each
+// line length and 6608 bytes per pass.  It does not move with what the kernels keep besides (stages' own
+// twiddle tables, tables of q^2, larger descriptors), so that the plans this entry point takes stay the same;
+// the array's room for them is twice the limit.  (A pass's tables of q^2 are half as long as its factors, a
+// length's twiddle tables at most twice as long as the line.)
+static size_t const_points(const Planner& pl)
+{
+    size_t n = pl.tables.size();
+    std::set<int> lengths;
+    for (const KernelDesc& k : pl.kernels) {
+        if (k.kind != K_LINE) continue;
+        if (k.line.ang) n -= (size_t)(k.line.nx + 1) / 2 + (size_t)(k.line.nz + 1) / 2;
+        lengths.insert(k.line.axis == 0 ? k.line.nx : k.line.nz);
+    }
+    auto pad = [&]() { n = (n + 31) & ~(size_t)31; };          // (each part starts on 256 bytes)
+    pad();
+    n += pl.kernels.size() * 6608 / sizeof(float2);
+    for (int N : lengths) {
+        pad();
+        n += N;
+    }
+    return n;
 }
 
 }  // namespace srwg
@@ -136,8 +162,9 @@ extern "C" SRWG_API int srwgPropagElecFieldStatic(const SRWLWfr* pWfr, const SRW
         line_twiddles(N, tw);
         cst.insert(cst.end(), tw.begin(), tw.end());
     }
-    if (cst.size() > SRWG_STATIC_CONST_POINTS) {
-        set_last_detail("the plan's tables need " + std::to_string(cst.size()) + " points, above the static limit of " +
+    const size_t counted = const_points(pl);
+    if (counted > SRWG_STATIC_CONST_POINTS || cst.size() > SRWG_STATIC_CONST_ROOM) {
+        set_last_detail("the plan's tables need " + std::to_string(counted) + " points, above the static limit of " +
                         std::to_string(SRWG_STATIC_CONST_POINTS));
         return SRWG_ERR_STATIC_LIMIT;
     }
@@ -158,7 +185,7 @@ extern "C" SRWG_API int srwgPropagElecFieldStatic(const SRWLWfr* pWfr, const SRW
     cudaStream_t st = (cudaStream_t)stream;
     float2* work = base;
     float2* cdev = base + 4 * (size_t)SRWG_STATIC_WORK_POINTS;
-    double* mom = (double*)(cdev + SRWG_STATIC_CONST_POINTS);     // slots | scratch
+    double* mom = (double*)(cdev + SRWG_STATIC_CONST_ROOM);     // slots | scratch
     cudaError_t e = cudaMemcpyAsync(cdev, cst.data(), cst.size() * sizeof(float2), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) { set_last_detail(std::string("constant upload: ") + cudaGetErrorString(e)); return SRWG_ERR_CUDA; }
     const KernelDesc* gk = (const KernelDesc*)(cdev + descOff);
