@@ -365,28 +365,36 @@ template <int R> __device__ __forceinline__ void pdft(P2* v)
     else pdodd<R>(v);
 }
 
-// twiddles of a stage: w, w^2, w^4, w^8 from its table (entry m of each of its rows of `pitch` entries),
-// loaded before the butterfly's inputs; v_k *= w^k, the other powers as their products
-struct TwP {
-    float2 w[4];
+// twiddles of a stage: v_k *= w^k from its table (entry m of each of its rows of `pitch` entries), loaded before the
+// butterfly's inputs.  A product of two table entries has their roundings and its own: with products of up to
+// four entries (1, 2, 4, 8) at every radix, propagations between drifts at 64^2, 256^2, 512^2 and 2048^2 were
+// 4.0, 4.8, 3.8 and 5.0e-7 off in 64 bits, with the rows of tw_power 2.9, 3.1, 2.5 and 3.9e-7, in the same
+// time (at 2240 x 1536, where registers are short, 216 instead of 212 us).
+template <int R> struct TwP {
+    float2 w[tw_rows(R)];
 };
-template <int R> __device__ __forceinline__ TwP ptwload(const float2* __restrict__ tw, int m, int pitch)
+template <int R> __device__ __forceinline__ TwP<R> ptwload(const float2* __restrict__ tw, int m, int pitch)
 {
-    TwP p;
+    TwP<R> p;
 #pragma unroll
-    for (int e = 0; e < 4; e++)
-        if ((1 << e) < R) p.w[e] = __ldg(&tw[m + e * pitch]);
+    for (int e = 0; e < tw_rows(R); e++) p.w[e] = __ldg(&tw[m + e * pitch]);
     return p;
 }
-template <int R> __device__ __forceinline__ void ptwiddle(P2* v, const TwP& p)
+template <int R> __device__ __forceinline__ void ptwiddle(P2* v, const TwP<R>& p)
 {
 #pragma unroll
     for (int r = 1; r < R; r++) {
-        float2 w = make_float2(1.f, 0.f);
-        bool first = true;
+        float2 w;
+        if constexpr (R <= 8) {
+            w = p.w[r - 1];
+        } else if constexpr (R == 16) {
+            w = r < 4 ? p.w[r - 1] : r % 4 == 0 ? p.w[r / 4 + 2] : cmul(p.w[r % 4 - 1], p.w[r / 4 + 2]);
+        } else {
+            bool first = true;
 #pragma unroll
-        for (int e = 0; e < 4; e++)
-            if (r & (1 << e)) { w = first ? p.w[e] : cmul(w, p.w[e]); first = false; }
+            for (int e = 0; e < 4; e++)
+                if (r & (1 << e)) { w = first ? p.w[e] : cmul(w, p.w[e]); first = false; }
+        }
         v[r] = pmul(v[r], w);
     }
 }
@@ -701,7 +709,7 @@ __device__ __forceinline__ void run_first(const Z& z, float4* s, const PLine& x,
     const int L1 = z.L(1);
 #pragma unroll 1
     for (int j = t; j < L1; j += z.T()) {
-        const TwP wp = ptwload<R>(tw + z.tw1(0), j, L1);
+        const TwP<R> wp = ptwload<R>(tw + z.tw1(0), j, L1);
         P2 v[R];
         pload<R, COLS, EXTRA, VEC>(v, x, c, j, L1, z.N(), cj);
         pdft<R>(v);
@@ -722,7 +730,7 @@ __device__ __forceinline__ void run_mid(const Z& z, int st, float4* s, const flo
     for (int b = t; b < nb; b += z.T()) {
         int w, o;
         float4* a = s + place_mid(z, st, b, w, o);
-        const TwP wp = ptwload<R>(tb, FWD ? o : low_index(z, st, w), tp);
+        const TwP<R> wp = ptwload<R>(tb, FWD ? o : low_index(z, st, w), tp);
         P2 v[R];
 #pragma unroll
         for (int r = 0; r < R; r++) v[r] = lds2(a + r * Ls);
@@ -758,7 +766,7 @@ __device__ __forceinline__ void run_turn(const Z& z, float4* s, const PLine& x, 
 #pragma unroll 1
     for (int u = t; u < M; u += z.T()) {
         float4* a = s + place_last(z, u);
-        const TwP wp = ptwload<R>(tw + z.tw2(z.n() - 1), u, M);
+        const TwP<R> wp = ptwload<R>(tw + z.tw2(z.n() - 1), u, M);
         P2 v[R];
 #pragma unroll
         for (int r = 0; r < R; r++) v[r] = lds2(a + r);

@@ -50,8 +50,10 @@ struct PShape {
     SRWG_HD int divB(int u, int s) const { return qdiv(u, dB[s]); }
 };
 
-// rows of a stage's twiddle table: the powers 1, 2, 4, 8 below the radix
-SRWG_HD constexpr int tw_rows(int R) { return R > 8 ? 4 : R > 4 ? 3 : R > 2 ? 2 : 1; }
+// rows of a stage's twiddle table: every power below the radix up to radix 8; 1, 2, 3, 4, 8, 12 for radix 16 (any other
+// is the product of two of them); 1, 2, 4, 8 for those between (up to three factors)
+SRWG_HD constexpr int tw_rows(int R) { return R == 16 ? 6 : R > 8 ? 4 : R - 1; }
+SRWG_HD constexpr int tw_power(int R, int row) { return R == 16 ? (row < 4 ? row + 1 : 4 * (row - 2)) : R > 8 ? 1 << row : row + 1; }
 
 template <int R0, int R1, int R2, int R3, int TT> struct FShape {
     static constexpr bool fixed = true;
@@ -265,23 +267,23 @@ inline bool make_pair_shape(int N, PairShape& z)
     return true;
 }
 
-// the twiddle tables of a schedule: for stage s of the first transform W_(L[s])^(o 2^e), o < L[s + 1], for
-// digit s of the second one W_(R[0] .. R[s])^(u 2^e), u < R[0] .. R[s - 1]; a row per e.  (FP64, rounded)
+// the twiddle tables of a schedule: for stage s of the first transform W_(L[s])^(o e), o < L[s + 1], for digit s
+// of the second one W_(R[0] .. R[s])^(u e), u < R[0] .. R[s - 1]; a row per power e (tw_power).  (FP64, rounded)
 template <class F2> inline void fill_twiddles(const PairShape& z, std::vector<F2>& h)
 {
     h.resize(z.twLen);
-    auto put = [&](int off, int rows, int n, int period) {
-        for (int e = 0; e < rows; e++)
+    auto put = [&](int off, int R, int n, int period) {
+        for (int e = 0; e < tw_rows(R); e++)
             for (int k = 0; k < n; k++) {
-                const double a = -2. * M_PI * (double)(((long long)k << e) % period) / (double)period;
+                const double a = -2. * M_PI * (double)((long long)k * tw_power(R, e) % period) / (double)period;
                 F2& v = h[off + e * n + k];
                 v.x = (float)cos(a);
                 v.y = (float)sin(a);
             }
     };
     const int N = z.len[0];
-    for (int s = 0; s + 1 < z.n; s++) put(z.tw1[s], tw_rows(z.R[s]), z.len[s + 1], z.len[s]);
-    for (int s = z.n - 1; s >= 1; s--) put(z.tw2[s], tw_rows(z.R[s]), N / z.len[s], N / z.len[s + 1]);
+    for (int s = 0; s + 1 < z.n; s++) put(z.tw1[s], z.R[s], z.len[s + 1], z.len[s]);
+    for (int s = z.n - 1; s >= 1; s--) put(z.tw2[s], z.R[s], N / z.len[s], N / z.len[s + 1]);
 }
 
 }  // namespace srwg
