@@ -368,8 +368,9 @@ template <int R> __device__ __forceinline__ void pdft(P2* v)
 // twiddles of a stage: v_k *= w^k from its table (entry m of each of its rows of `pitch` entries), loaded before the
 // butterfly's inputs.  A product of two table entries has their roundings and its own: with products of up to
 // four entries (1, 2, 4, 8) at every radix, propagations between drifts at 64^2, 256^2, 512^2 and 2048^2 were
-// 4.0, 4.8, 3.8 and 5.0e-7 off in 64 bits, with the rows of tw_power 2.9, 3.1, 2.5 and 3.9e-7, in the same
-// time (at 2240 x 1536, where registers are short, 216 instead of 212 us).
+// 4.0, 4.8, 3.8 and 4.9e-7 off in 64 bits, with the rows of tw_power 2.9, 3.1, 2.5 and 4.2e-7, for 0 to 2 %
+// of the time (512^2 30.5 us either way, 2048^2 211 to 213, 2240 x 1536, where registers are short, 212 to
+// 215).  A sixth row for radix 16 (power 3) gives 3.9e-7 at 2048^2 and takes 221 us.
 template <int R> struct TwP {
     float2 w[tw_rows(R)];
 };
@@ -388,7 +389,9 @@ template <int R> __device__ __forceinline__ void ptwiddle(P2* v, const TwP<R>& p
         if constexpr (R <= 8) {
             w = p.w[r - 1];
         } else if constexpr (R == 16) {
-            w = r < 4 ? p.w[r - 1] : r % 4 == 0 ? p.w[r / 4 + 2] : cmul(p.w[r % 4 - 1], p.w[r / 4 + 2]);
+            const float2 lo = r % 4 == 3 ? cmul(p.w[0], p.w[1]) : p.w[r % 4 == 2];
+            const float2 hi = r / 4 == 3 ? p.w[4] : p.w[r / 4 == 2 ? 3 : 2];
+            w = r < 4 ? lo : r % 4 == 0 ? hi : cmul(lo, hi);
         } else {
             bool first = true;
 #pragma unroll

@@ -50,10 +50,10 @@ struct PShape {
     SRWG_HD int divB(int u, int s) const { return qdiv(u, dB[s]); }
 };
 
-// rows of a stage's twiddle table: every power below the radix up to radix 8; 1, 2, 3, 4, 8, 12 for radix 16 (any other
-// is the product of two of them); 1, 2, 4, 8 for those between (up to three factors)
-SRWG_HD constexpr int tw_rows(int R) { return R == 16 ? 6 : R > 8 ? 4 : R - 1; }
-SRWG_HD constexpr int tw_power(int R, int row) { return R == 16 ? (row < 4 ? row + 1 : 4 * (row - 2)) : R > 8 ? 1 << row : row + 1; }
+// rows of a stage's twiddle table: every power below the radix up to radix 8; 1, 2, 4, 8 above it (the others are
+// products), and 12 for radix 16
+SRWG_HD constexpr int tw_rows(int R) { return R == 16 ? 5 : R > 8 ? 4 : R - 1; }
+SRWG_HD constexpr int tw_power(int R, int row) { return R <= 8 ? row + 1 : row < 4 ? 1 << row : 12; }
 
 template <int R0, int R1, int R2, int R3, int TT> struct FShape {
     static constexpr bool fixed = true;
