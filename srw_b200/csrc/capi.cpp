@@ -118,16 +118,15 @@ int device_twiddles(DeviceCtx& c, int N, const float2** out)
 }
 
 // ------------------------------------------------------------------------------------------------
-// autotuned launch shapes: kernel family and lines per CTA of the compile-time-length line kernels
-// per (axis, N), measured by srw_b200.tune and stored as lines "rows|cols N L [spec]" in
-// models/line_tuning.txt next to the library (or the file named by SRWG_TUNING); "spec" selects the
-// specialised kernel for a power of two.  srwgTuneSetLines / srwgTuneSetFamily change entries at
-// run time.
+// autotuned launch shapes: lines per CTA per (axis, N), measured by srw_b200.tune and stored as lines
+// "rows|cols N L [spec]" in models/line_tuning.txt next to the library (or the file named by SRWG_TUNING);
+// srwgTuneSetLines changes entries at run time.  The class of a length (power of two, or "spec": general) bounds
+// the lines an entry may have (fixed_lines_valid) and chooses no kernel.
 // ------------------------------------------------------------------------------------------------
 static std::mutex g_tuneMutex;
 struct TuneEntry {
-    int fam = 0;       // 0: the default family of the length
-    int lines = 0;     // 0: the family's default lines per CTA
+    int fam = 0;       // 0: the length's own class
+    int lines = 0;     // 0: the built-in choice
 };
 static std::map<std::pair<int, int>, TuneEntry> g_tune;
 static bool g_tuneLoaded = false;
@@ -195,15 +194,6 @@ int fixed_family(int axis, int N)
     return e.fam ? e.fam : default_family(N);
 }
 
-int fixed_lines_per_cta(int axis, int N)
-{
-    const int fam = fixed_family(axis, N);
-    if (fam != FAM_POW2 && fam != FAM_SPEC) return 0;
-    const TuneEntry e = tuned(axis, N);
-    if (e.lines > 0 && fixed_lines_valid(axis, N, e.lines, fam)) return e.lines;
-    return fam == FAM_POW2 ? line2_lines_per_cta(axis, N) : linen_lines_per_cta(axis, N);
-}
-
 // pairs of lines per CTA: the tuned lines halved, else about 256 threads (columns: at least two pairs,
 // 32-byte pieces of a row, a power of two)
 static int pairs_per_cta(int axis, int N, const PairShape& z)
@@ -218,6 +208,13 @@ static int pairs_per_cta(int axis, int N, const PairShape& z)
     }
     while (G > 1 && (G * z.T > 512 || (size_t)G * (z.slot + 8) * 16 > SRWG_LINE_SMEM_MAX)) G = axis == 1 ? G / 2 : G - 1;
     return G;
+}
+
+int fixed_lines_per_cta(int axis, int N)
+{
+    if (default_family(N) == 0) return 0;
+    const PairShape* z = pair_shape(N);
+    return z ? 2 * pairs_per_cta(axis, N, *z) : 1;
 }
 
 int pair_block(int N, int nl)

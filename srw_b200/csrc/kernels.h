@@ -11,31 +11,14 @@ namespace srwg {
 // dynamic shared memory of a line pass (leaves room for the static descriptor copy)
 #define SRWG_LINE_SMEM_MAX (220 * 1024)
 
-// shared-memory pitch of a line of N points in the line passes: one pad point per 16 (conflict-free
-// Stockham exchanges), then rounded up so that the lines of a column tile start 32 / L banks apart
-// (a half-warp of a column pass reads 16 / L points of each of L lines, 8 bytes each: together 32
-// distinct banks): P = 16 / L modulo 16 points for L = 2, 4, 8, 1 for L >= 16; rows (their lanes
-// stay within one line) and L = 1: 4 modulo 16, which keeps every slot 16-byte aligned for the
-// bulk copies of row tiles
+// shared-memory pitch of a line of N points in the pass of 16384 (line2.cuh): one pad point per 16 (conflict-free
+// Stockham exchanges), a multiple of 16 bytes; with L lines as the tuning entry points' bound on entries (a
+// column tile's lines 32 / L banks apart)
 inline size_t line_pitch(int N, int L = 1, bool cols = false)
 {
     const size_t P = (size_t)N + N / 16;
     const size_t r = (cols && L >= 2) ? (L >= 16 ? 1 : 16 / L) : 4;
     return P + ((r + 16 - P % 16) % 16);
-}
-
-// lines per CTA of the power-of-two line pass (line2_kernel): rows ~256 threads, columns up to
-// 1024 threads (at most 32 columns), within the shared-memory budget; pitch N + N/16 + 4 points.
-// (Column tiles of half the width, two CTAs per SM, measured slower: the row pass then writes
-// 16-byte pieces per row and column block, and the column pass's stores are half sectors.)
-inline int line2_lines_per_cta(int axis, int N)
-{
-    const int T = N / 16;
-    int L = axis == 0 ? 256 / T : 1024 / T;
-    if (L < 1) L = 1;
-    if (axis == 1 && L > 32) L = 32;
-    while (L > 1 && (size_t)L * line_pitch(N, L, axis == 1) * 8 > SRWG_LINE_SMEM_MAX) L--;
-    return L;
 }
 
 // what a line pass kernel takes (its descriptor stays in device memory)
@@ -191,7 +174,7 @@ inline bool linen_pow2(int N)
 #undef SRWG_LINEN_IS
     return false;
 }
-// lengths of the passes on pairs of lines: every even 2^a 3^b 5^c 7^d 11^e 13^f (e, f <= 1) from 4 to
+// lengths of the passes on pairs of lines: every even 2^a 3^b 5^c 7^d 11^e 13^f from 4 to
 // 8192 (they take zero windows and column blocks, and write intensities)
 bool pair_supported(int N);
 // the twiddle tables of a line pass of N points, as its kernel reads them
@@ -199,27 +182,9 @@ void line_twiddles(int N, std::vector<float2>& h);
 // columns that a column pass of N points transforms per CTA on a grid of nl columns: the width of
 // the column blocks the row pass before it writes (0: the pass is not one on pairs, or nl has no such blocks)
 int pair_block(int N, int nl);
-// kernel families of the tuning entry points
-enum { FAM_TAB = 0, FAM_POW2 = 1, FAM_GEN = 2, FAM_SPEC = 3 };
-// lines per CTA of the specialised general-length pass (at most 512 threads, 128 registers each):
-// rows up to 512 threads, columns a power of two up to 512 threads / 32 columns (the column-block
-// width of the row pass before it), within the shared-memory budget; T = ceil(N/16) threads per
-// line, pitch N + N/16 + 4 points
-inline int linen_lines_per_cta(int axis, int N)
-{
-    const int T = (N + 15) / 16;
-    int L;
-    if (axis == 0) {
-        L = 512 / T;
-        if (L < 1) L = 1;
-    } else {
-        L = 1;
-        while (2 * L * T <= 512 && 2 * L <= 32) L *= 2;
-    }
-    while (L > 1 && (size_t)L * line_pitch(N, L, axis == 1) * 8 > SRWG_LINE_SMEM_MAX) L = axis == 0 ? L - 1 : L / 2;
-    return L;
-}
-// whether L lines per CTA is a valid launch shape of kernel family fam for length N
+// classes of tuned lengths (the tuning entry points' families)
+enum { FAM_POW2 = 1, FAM_SPEC = 3 };
+// whether the tuning entry points take L lines per CTA for length N of class fam
 inline bool fixed_lines_valid(int axis, int N, int L, int fam)
 {
     if (L < 1 || (size_t)L * line_pitch(N, L, axis == 1) * 8 > SRWG_LINE_SMEM_MAX) return false;
@@ -228,8 +193,8 @@ inline bool fixed_lines_valid(int axis, int N, int L, int fam)
     if (fam == FAM_SPEC && (linen_supported(N) || linen_pow2(N))) return ((N + 15) / 16) * L <= 512;
     return false;
 }
-// family and lines per CTA of the tuned lengths: the tuning table's choice where it has one
-// (capi.cpp), else the defaults above; lines 0 for other lengths
+// class of a tuned length, and the lines per CTA its passes are launched with (whole pairs; fewer where a launch has
+// few lines, as many as its blocks where it reads blocks of lines; 0 for other lengths)
 int fixed_family(int axis, int N);
 int fixed_lines_per_cta(int axis, int N);
 cudaError_t launch_resize(const ResizeLaunch& p, cudaStream_t st);

@@ -61,7 +61,7 @@ def line_pitch(n, lines=1, cols=False):
     p = n + n // 16
     r = (1 if lines >= 16 else 16 // lines) if (cols and lines >= 2) else 4
     return p + (r + 16 - p % 16) % 16
-POW2_SPEC = [256, 512, 1024, 2048, 4096, 8192]       # powers of two the specialised pass is built for
+POW2_SPEC = [256, 512, 1024, 2048, 4096, 8192]       # powers of two whose entries may be of either class
 
 
 def families(n):
@@ -71,9 +71,9 @@ def families(n):
 
 
 def launch_shape(axis, n):
-    """(kernel family name, lines per CTA) the library uses for a line pass of n points along axis 0
-    (rows) or 1 (columns): the tuning table's entry, else its defaults; (None, 0) for lengths that
-    run the run-time-scheduled pass."""
+    """(class name, lines per CTA) of the line passes of n points along axis 0 (rows) or 1 (columns): 'pow2' or
+    'spec' (a tuned general length) and the whole pairs of lines a CTA of the library takes, the tuning table's
+    or its own choice; (None, 0) for other lengths.  (A launch of few lines takes fewer.)"""
     L = capi.lib()
     fam, lines = C.c_int(), C.c_int()
     capi.check(L.srwgTuneGetFamily(int(axis), int(n), C.byref(fam)), 'tune family')

@@ -19,3 +19,19 @@ def test_table_holds_whole_pairs():
         assert lines % 2 == 0 and lines // 2 * threads[n] <= 512, (axis, n, lines)
         if axis == 'cols':
             assert lines >= 4 and lines & (lines - 1) == 0, (n, lines)      # 32-byte pieces of a row
+
+
+def test_reported_lines_are_whole_pairs():
+    """The lines per CTA that the library reports are those it launches: two per pair, also where an entry is odd."""
+    import ctypes as C
+    from srw_b200 import capi
+    L = capi.lib()
+    got = C.c_int()
+    try:
+        for axis, n, lines, want in ((0, 2240, 1, 2), (0, 2240, 2, 2), (0, 2240, 3, 2), (0, 512, 7, 6), (1, 512, 1, 2),
+                                     (1, 512, 8, 8), (0, 2240, 0, 2), (1, 2240, 0, 4), (0, 4096, 0, 2), (1, 4096, 0, 4)):
+            assert L.srwgTuneSetLines(axis, n, lines) == 0
+            assert L.srwgTuneGetLines(axis, n, C.byref(got)) == 0
+            assert got.value == want, (axis, n, lines)
+    finally:
+        L.srwgTuneLoad(tune.TXT.encode(), None)
