@@ -1,4 +1,4 @@
-// Device helpers shared by the pass kernels (included by kernels.cu and the line2_*.cu units).
+// Device helpers shared by the pass kernels (included by kernels.cu, linep.cuh and line2.cuh).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -20,7 +20,6 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b)
 // complex add / subtract as one packed FP32x2 instruction each (sm_100); b * (-1) + a is exactly a - b
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
-__device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
 // multiply by -i (forward, DIR=+1) or +i (inverse, DIR=-1)
 template <int DIR> __device__ __forceinline__ float2 mul_mi(float2 a)
 {
@@ -44,14 +43,8 @@ __device__ __forceinline__ float2 expi(double ph)
 }
 
 // ------------------------------------------------------------------------------------------------
-// small DFTs (DIR=+1: exp(-2 pi i nk/R) like FFTW_FORWARD; DIR=-1: exp(+...) like FFTW_BACKWARD)
+// small DFTs of the pass of 16384 points (DIR=+1: exp(-2 pi i nk/R) like FFTW_FORWARD; DIR=-1: exp(+...) like FFTW_BACKWARD)
 // ------------------------------------------------------------------------------------------------
-template <int DIR> __device__ __forceinline__ void dft2(float2* v)
-{
-    float2 a = v[0];
-    v[0] = cadd(a, v[1]);
-    v[1] = csub(a, v[1]);
-}
 template <int DIR> __device__ __forceinline__ void dft4(float2& v0, float2& v1, float2& v2, float2& v3)
 {
     float2 a0 = cadd(v0, v2), a1 = csub(v0, v2), a2 = cadd(v1, v3), a3 = mul_mi<DIR>(csub(v1, v3));
@@ -61,23 +54,6 @@ template <int DIR> __device__ __forceinline__ void dft4(float2& v0, float2& v1, 
     v3 = csub(a1, a3);
 }
 template <int DIR> __device__ __forceinline__ void dft4(float2* v) { dft4<DIR>(v[0], v[1], v[2], v[3]); }
-
-template <int DIR> __device__ __forceinline__ void dft8(float2* v)
-{
-    const float h = 0.70710678118654752440f;
-    float2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6];
-    float2 o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
-    dft4<DIR>(e0, e1, e2, e3);
-    dft4<DIR>(o0, o1, o2, o3);
-    // W8^1 = (1 -/+ i)/sqrt2, W8^2 = -/+ i, W8^3 = (-1 -/+ i)/sqrt2
-    float2 t1 = make_float2(h * (o1.x + (DIR > 0 ? o1.y : -o1.y)), h * (o1.y - (DIR > 0 ? o1.x : -o1.x)));
-    float2 t2 = mul_mi<DIR>(o2);
-    float2 t3 = make_float2(h * (-o3.x + (DIR > 0 ? o3.y : -o3.y)), h * (-o3.y - (DIR > 0 ? o3.x : -o3.x)));
-    v[0] = cadd(e0, o0); v[4] = csub(e0, o0);
-    v[1] = cadd(e1, t1); v[5] = csub(e1, t1);
-    v[2] = cadd(e2, t2); v[6] = csub(e2, t2);
-    v[3] = cadd(e3, t3); v[7] = csub(e3, t3);
-}
 
 template <int DIR> __device__ __forceinline__ void dft16(float2* v)
 {
@@ -106,81 +82,11 @@ template <int DIR> __device__ __forceinline__ void dft16(float2* v)
     }
 }
 
-template <int DIR> __device__ __forceinline__ void dft3(float2* v)
+template <int R, int DIR> __device__ __forceinline__ void dftR(float2* v)
 {
-    const float s = 0.86602540378443864676f;
-    float2 t1 = cadd(v[1], v[2]);
-    float2 t2 = make_float2(v[0].x - 0.5f * t1.x, v[0].y - 0.5f * t1.y);
-    float2 t3 = mul_mi<DIR>(cscale(csub(v[1], v[2]), s));
-    v[0] = cadd(v[0], t1);
-    v[1] = cadd(t2, t3);
-    v[2] = csub(t2, t3);
-}
-
-template <int DIR> __device__ __forceinline__ void dft5(float2* v)
-{
-    const float c1 = 0.30901699437494742410f, c2 = -0.80901699437494742410f;
-    const float s1 = 0.95105651629515357212f, s2 = 0.58778525229247312917f;
-    float2 t1 = cadd(v[1], v[4]), t2 = cadd(v[2], v[3]), t3 = csub(v[1], v[4]), t4 = csub(v[2], v[3]);
-    float2 a1 = make_float2(v[0].x + c1 * t1.x + c2 * t2.x, v[0].y + c1 * t1.y + c2 * t2.y);
-    float2 a2 = make_float2(v[0].x + c2 * t1.x + c1 * t2.x, v[0].y + c2 * t1.y + c1 * t2.y);
-    float2 b1 = mul_mi<DIR>(make_float2(s1 * t3.x + s2 * t4.x, s1 * t3.y + s2 * t4.y));
-    float2 b2 = mul_mi<DIR>(make_float2(s2 * t3.x - s1 * t4.x, s2 * t3.y - s1 * t4.y));
-    v[0] = cadd(v[0], cadd(t1, t2));
-    v[1] = cadd(a1, b1); v[4] = csub(a1, b1);
-    v[2] = cadd(a2, b2); v[3] = csub(a2, b2);
-}
-
-// 7-point DFT from the symmetric pairs (v_k +/- v_(7-k)): 36 real multiply-adds, no table
-template <int DIR> __device__ __forceinline__ void dft7(float2* v)
-{
-    const float c1 = 0.62348980185873353053f, c2 = -0.22252093395631440429f, c3 = -0.90096886790241912624f;
-    const float s1 = 0.78183148246802980871f, s2 = 0.97492791218182360702f, s3 = 0.43388373911755812048f;
-    const float2 a1 = cadd(v[1], v[6]), a2 = cadd(v[2], v[5]), a3 = cadd(v[3], v[4]);
-    const float2 b1 = csub(v[1], v[6]), b2 = csub(v[2], v[5]), b3 = csub(v[3], v[4]);
-    const float2 x0 = v[0];
-    auto lin = [&](float p, float q, float r, float2 u1, float2 u2, float2 u3, float2 z) {
-        return make_float2(fmaf(p, u1.x, fmaf(q, u2.x, fmaf(r, u3.x, z.x))), fmaf(p, u1.y, fmaf(q, u2.y, fmaf(r, u3.y, z.y))));
-    };
-    const float2 z0 = make_float2(0.f, 0.f);
-    const float2 A1 = lin(c1, c2, c3, a1, a2, a3, x0), B1 = mul_mi<DIR>(lin(s1, s2, s3, b1, b2, b3, z0));
-    const float2 A2 = lin(c2, c3, c1, a1, a2, a3, x0), B2 = mul_mi<DIR>(lin(s2, -s3, -s1, b1, b2, b3, z0));
-    const float2 A3 = lin(c3, c1, c2, a1, a2, a3, x0), B3 = mul_mi<DIR>(lin(s3, -s1, s2, b1, b2, b3, z0));
-    v[0] = cadd(x0, cadd(a1, cadd(a2, a3)));
-    v[1] = cadd(A1, B1); v[6] = csub(A1, B1);
-    v[2] = cadd(A2, B2); v[5] = csub(A2, B2);
-    v[3] = cadd(A3, B3); v[4] = csub(A3, B3);
-}
-
-// generic odd radix (7, 11, 13): direct O(R^2) DFT; W_R^m = tw[m * N / R]
-template <int R, int DIR> __device__ __forceinline__ void dftg(float2* v, const float2* __restrict__ tw, int NdR)
-{
-    float2 o[R];
-#pragma unroll
-    for (int m = 0; m < R; m++) {
-        float2 acc = v[0];
-#pragma unroll
-        for (int n = 1; n < R; n++) {
-            float2 w = __ldg(&tw[((n * m) % R) * NdR]);
-            if (DIR < 0) w.y = -w.y;
-            acc = cadd(acc, cmul(v[n], w));
-        }
-        o[m] = acc;
-    }
-#pragma unroll
-    for (int m = 0; m < R; m++) v[m] = o[m];
-}
-
-template <int R, int DIR> __device__ __forceinline__ void dftR(float2* v, const float2* __restrict__ tw, int N)
-{
-    if (R == 2) dft2<DIR>(v);
-    else if (R == 3) dft3<DIR>(v);
-    else if (R == 4) dft4<DIR>(v);
-    else if (R == 5) dft5<DIR>(v);
-    else if (R == 8) dft8<DIR>(v);
-    else if (R == 16) dft16<DIR>(v);
-    else if (R == 7) dft7<DIR>(v);
-    else dftg<R, DIR>(v, tw, N / R);
+    static_assert(R == 4 || R == 16, "stages of 16384 points");
+    if constexpr (R == 4) dft4<DIR>(v);
+    else dft16<DIR>(v);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -190,34 +96,6 @@ template <int R, int DIR> __device__ __forceinline__ void dftR(float2* v, const 
 __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
-
-// accumulates phase, complex factor and zeroing of PwOps at kernel index (i, j)
-__device__ __forceinline__ void pw_eval(const PwOps& pw, int i, int j, double& ph, float2& f, bool& zero)
-{
-    if (pw.has_quad) {
-        double di = (double)i, dj = (double)j;
-        ph += fma(fma(pw.Ai, di, pw.Bi), di, fma(fma(pw.Aj, dj, pw.Bj), dj, pw.C));
-    }
-    if (pw.has_ang) {
-        double qx = pw.qx0 + (double)i * pw.dqx, qz = pw.qz0 + (double)j * pw.dqz;
-        double q2 = qx * qx + qz * qz;
-        double c1q2 = pw.c1 * q2;
-        ph += pw.c0 * q2 * (1. + c1q2 + 2. * c1q2 * c1q2);
-    }
-    if (pw.has_scale) f = cmul(f, make_float2(pw.sre, pw.sim));
-    for (int m = 0; m < pw.nmask; m++) {
-        const PwMask& k = pw.mask[m];
-        double x = dadd(k.x0, dmul((double)i, k.dx));
-        double z = dadd(k.z0, dmul((double)j, k.dz));
-        double xr = dsub(x, k.cx), zr = dsub(z, k.cz);
-        bool outside;
-        if (k.type == 1) outside = (xr < -k.hx) || (xr > k.hx) || (zr < -k.hz) || (zr > k.hz);
-        else outside = dadd(dmul(xr, xr), dmul(zr, zr)) > k.r2;
-        zero |= k.obstacle ? !outside : outside;
-    }
-}
-
-__device__ __forceinline__ void extra_eval(const PwOps& e, int i, int j, float2& f, bool& zero, const float2* tabs);
 
 // RadPointModifier_PropToWaistBeyondParax (sroptdrf.h:712-754): exp(i k L (sqrt(1 + X) - 1)), or with
 // k L sqrt(1 + X) on the path-length option, X = -lambda^2 (qx^2 + qz^2); the square root for

@@ -1,16 +1,17 @@
-// Power-of-two line pass templates (instantiated per line length in line2_*.cu).
+// Line pass of 16384 points, one line per thread (instantiated in line2_14.cu and line2e_14.cu; shorter lines:
+// linep.cuh).
 #pragma once
 #include "common.cuh"
 
 namespace srwg {
 
 // ------------------------------------------------------------------------------------------------
-// LINE pass, power-of-two lines (N >= 64): every thread owns 16 points of its line.  The first
+// LINE pass: every thread owns 16 points of its line.  The first
 // FFT stage reads its butterfly inputs straight from global memory through the point-wise chain
 // (coalesced: thread t reads t + T*m), the last stage writes straight to global memory through
 // the output chain; intermediate stages exchange through shared memory padded by one point per
-// 16 (conflict-free Stockham writes).  Complex adds and subtracts are packed FP32x2 instructions.  A second transform in the same pass (f1 -> f2) reads the
-// first one's output from shared memory through the middle chain.
+// 16 (conflict-free Stockham writes).  Complex adds and subtracts are packed FP32x2 instructions.  A second
+// transform in the same pass (f1 -> f2) reads the first one's output from shared memory through the middle chain.
 // ------------------------------------------------------------------------------------------------
 #define PADI(p) ((p) + ((p) >> 4))
 
@@ -86,7 +87,7 @@ __device__ __forceinline__ void stage16(float2* s, const float2* __restrict__ gi
     for (int b = 0; b < B; b++) {
         const int j = t + T * b;
         const int k = j & (NS - 1);
-        dftR<R, DIR>(v[b], tw, N);
+        dftR<R, DIR>(v[b]);
         const int base = (j / NS) * NS * R + k;
 #pragma unroll
         for (int r = 0; r < R; r++) {
