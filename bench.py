@@ -26,6 +26,7 @@ import json
 from array import array
 import math
 import os
+import re
 import statistics
 import subprocess
 import sys
@@ -47,15 +48,6 @@ PEAKS = os.path.join(HERE, 'MEASURED_PEAKS.json')
 BATCH = 16                                     # macro-electron wavefronts per step
 SIG = (30e-6, 5e-6, 5e-6, 2e-6)                # source: sigma x [m], x' [rad], y [m], y' [rad]
 SIG_E = 1e-3                                   # relative electron energy spread (photon energy E (1 + 2 d))
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch of a pass, from an ncu
-# capture of this workload (the plain passes' summary under profiles/); keyed by the pass tuple of
-# Plan.kernels().  Re-captured whenever the kernel changes.
-# (Not captured for the plain passes of the present kernels.)
-TRAFFIC = {}
-# the same per electron of the batched passes at the learned factors (ncu on a batch of 8); a launch
-# moves this times its electrons
-TRAFFIC_PER_ELECTRON = {('line_cols', 1536, 1600): (19659008 + 3882752) // 8,
-                        ('line_rows', 1536, 1600): (35271680 + 67584) // 8}
 
 
 # ------------------------------------------------------------------------------------------------
@@ -363,32 +355,68 @@ def hbm_peak():
     return 6650., 'fallback'
 
 
-def batched_passes(me, offs, stream, peak, peak_src, where):
-    """One batch of the multi-electron object `me` (MultiE) run without its graph, with CUDA events
-    around every pass (srwgMultiEAddTimed; adds the electrons): per-pass times and the roofline of the
-    dominant pass -- algorithmic bytes per electron (kernel_bytes; a last pass that writes the
-    intensity writes one float per point instead of two complex values) times the electrons of the
-    launch, over the pass's CUDA-event time."""
+def sampled_rows(acc, out):
+    """Rows of the output mesh `out` that a detector `acc` of rows two or more output rows apart reads: the two
+    around each of its rows that lies inside."""
+    y = np.linspace(acc.yStart, acc.yFin, int(acc.ny))
+    i = np.trunc((y - out['yStart']) * (out['ny'] - 1) / (out['yFin'] - out['yStart']) + 1e-9).astype(np.int64)
+    i = i[(i >= 0) & (i < out['ny'] - 1)]
+    return len(np.union1d(i, i + 1))
+
+
+def batch_bytes(me, nb, out):
+    """Algorithmic bytes of every pass of a launch of nb electrons of `me` (MultiE) from its shapes: what a pass
+    reads and writes of both components, windows only where passes leave out what is zero (the planner's
+    description of the base electron), the base field read once; a last pass that writes the intensity one
+    float per point, one that reads sampled rows only those (and so the column pass before it writes only
+    those) and the detector's FP64 sums once."""
+    lines = [l for l in me.describe().splitlines() if l.split()[1] in ('LINE', 'RESIZE')]
+    win = lambda l: [int(v) for p in re.findall(r'(?:lines=|points=)(-?\d+):(-?\d+)', l) for v in p]  # noqa: E731
+    step = (me._accm.yFin - me._accm.yStart) / (me.ny - 1)
+    rows = sampled_rows(me._accm, out)
+    res = []
+    for i, l in enumerate(lines):
+        f = l.split()
+        if f[1] == 'RESIZE':
+            nxo, nzo = map(int, f[2].split('x'))
+            x0, x1, z0, z1 = map(int, re.search(r'window=x(-?\d+):(-?\d+),z(-?\d+):(-?\d+)', l).groups())
+            res.append(16 * nxo * nzo + nb * 16 * (x1 - x0 + 1) * (z1 - z0 + 1))
+            continue
+        nx, nz = map(int, f[3].split('x'))
+        N, nl = (nx, nz) if f[2] == 'rows' else (nz, nx)
+        w = win(l)
+        wl, wp = (w[1] - w[0] + 1, w[3] - w[2] + 1) if w else (nl, N)
+        last = i + 1 == len(lines)
+        sampled = lambda q: ('intensity' in q and ' LINE rows' in q and  # noqa: E731
+                             step >= 2. * abs(out['yFin'] - out['yStart']) / (out['ny'] - 1))
+        read = 16 * wl * wp if i else 16 * wl * wp / nb
+        write = 16 * wl * N
+        if last and 'intensity' in l:
+            write = 4 * nl * N
+            if sampled(l):
+                read, write = 16 * rows * wp, 8. * me.nx * me.ny / nb
+        elif not last and sampled(lines[i + 1]) and f[2] == 'cols':
+            write = 16 * wl * rows
+        res.append(nb * (read + write))
+    return res
+
+
+def batched_passes(me, offs, stream, peak, peak_src, where, out):
+    """One batch of the multi-electron object `me` (MultiE, output mesh `out`) run without its graph, with CUDA
+    events around every pass (srwgMultiEAddTimed; adds the electrons): per-pass times and the roofline of the
+    dominant pass, algorithmic bytes (batch_bytes) over the pass's CUDA-event time."""
     ks, inten = me.info()
     ms = me.add_timed(offs, stream)
     nb = len(offs)
     per = ms[:len(ks)]
-    alg = [kernel_bytes(k) for k in ks]
-    if inten:
-        k = ks[-1]
-        alg[-1] = 2 * 8 * k[1] * k[2] + 4 * k[1] * k[2]
-        if k[0] == 'line_rows' and 2 * getattr(me, 'ny', k[2]) < k[2]:
-            # only rows around the detector's are read, and their sums are written: what is counted is the
-            # captured traffic where there is one, else two rows per detector row
-            t = TRAFFIC_PER_ELECTRON.get(tuple(k))
-            alg[-1] = t if t is not None else 2 * 8 * k[1] * 2 * me.ny
+    alg = batch_bytes(me, nb, out)
     kd = int(np.argmax(per))
-    achieved = alg[kd] * nb / (per[kd] / 1000.) / 1e9
+    achieved = alg[kd] / (per[kd] / 1000.) / 1e9
     return {"bound": "hbm", "kernel": "%s %s (batch of %d)" % (ks[kd][0], 'x'.join(map(str, ks[kd][1:])), nb),
             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_src,
-            "traffic": (TRAFFIC_PER_ELECTRON[tuple(ks[kd])] * nb if tuple(ks[kd]) in TRAFFIC_PER_ELECTRON else None),
-            "algorithmic_bytes": alg[kd] * nb, "avg_ms": float(per[kd]),
-            "per_pass_ms": [round(float(v), 4) for v in per], "accumulation_ms": round(float(ms[-1]), 4),
+            "traffic": None, "algorithmic_bytes": int(alg[kd]), "avg_ms": float(per[kd]),
+            "per_pass_ms": [round(float(v), 4) for v in per],
+            "per_pass_algorithmic_MB": [round(v / 1e6, 1) for v in alg], "accumulation_ms": round(float(ms[-1]), 4),
             "per_electron_ms": round(float(sum(ms)) / nb, 5), "passes": [list(k) for k in ks],
             "last_pass_writes_intensity": inten, "measured_on": where}
 
@@ -528,7 +556,8 @@ def measure_batched(args, dev, world, dist, factors=CONFIGURED, acc=None, e2e_le
     mean = acc_t.cpu().numpy() / n_all
     peak, peak_src = hbm_peak()
     passes = batched_passes(me, offs[0], stream.cuda_stream, peak, peak_src,
-                            "batched leg (configured factors), one batch of %d electrons, CUDA events per pass" % BATCH)
+                            "batched leg (configured factors), one batch of %d electrons, CUDA events per pass" % BATCH,
+                            Plan(w, bl, device=dev.index).output_mesh())
 
     # end to end through the public API: host offsets in, mean intensity (host) out, every step
     e2e = None
@@ -703,9 +732,11 @@ def measure_learned(args, dev, world, dist, acc):
                        "offsets from host, the run-time check included) + CheckedMultiE.mean (D2H of the %dx%d FP64 "
                        "mean intensity)" % (acc['nx'], acc['ny'])}
     peak, peak_src = hbm_peak()
-    passes = batched_passes(cm.safe if cm.fell_back else cm.fast, offs[0][:LEARNED_LAUNCH], stream.cuda_stream, peak,
-                            peak_src, "learned leg, one launch of %d electrons, CUDA events per pass" % LEARNED_LAUNCH)
     from srw_b200.plan import Plan
+    passes = batched_passes(cm.safe if cm.fell_back else cm.fast, offs[0][:LEARNED_LAUNCH], stream.cuda_stream, peak,
+                            peak_src, "learned leg, one launch of %d electrons, CUDA events per pass" % LEARNED_LAUNCH,
+                            Plan(w, beamline_objs(mod, learned.CONSERVATIVE if cm.fell_back else factors),
+                                 device=dev.index).output_mesh())
     nk_f = Plan(w, beamline_objs(mod, factors), device=dev.index).n_kernels
     nk_c = Plan(w, beamline_objs(mod), device=dev.index).n_kernels
     return {"value": value, "unit": UNIT, "ms_per_step": total_ms / args.steps, "batch": LEARNED_BATCH,
@@ -933,7 +964,7 @@ def roofline(pl, peak, peak_src, where):
     achieved = alg / (per_k[kd] / 1000.) / 1e9
     return {"bound": "hbm", "kernel": "%s %s" % (kinfo[kd][0], 'x'.join(map(str, kinfo[kd][1:]))),
             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_src,
-            "traffic": TRAFFIC.get(kinfo[kd]), "algorithmic_bytes": alg, "avg_ms": float(per_k[kd]),
+            "traffic": None, "algorithmic_bytes": alg, "avg_ms": float(per_k[kd]),
             "per_pass_ms": [round(float(v), 4) for v in per_k], "passes": [list(k) for k in kinfo],
             "measured_on": where}
 
