@@ -43,16 +43,17 @@ struct GemmTail {
     float* bsum;
 };
 
-// op(A) is M x K (A row-major, lda; transposed when TA), op(B) is K x N.  A CTA makes a 32 x 64 tile over
-// one of gridDim.z pieces of K (steps of 32, the next step's operands loaded while this one is
-// multiplied); the pieces are the CTAs of a cluster, which then add their tiles through distributed
-// shared memory in piece order (no workspace, no atomics: the sum does not depend on scheduling).
+// op(A) is M x K (A row-major, lda; transposed when TA), op(B) is K x N.  A CTA makes a GM x 64 tile over one of
+// gridDim.z pieces of K (steps of 32, the next step's operands loaded while this one is multiplied); the pieces
+// are the CTAs of a cluster, which then add their tiles through distributed shared memory in piece order (no
+// workspace, no atomics: the sum does not depend on scheduling); one piece writes its tile from registers.
 // The network's products are small and long: 128 x 256 with K = 4109 is 8 tiles of 64 x 64, whose 257
-// serial steps took 385 us; 16 tiles in 8 pieces occupy 128 SMs with 17 steps each.
-#define GM 32
+// serial steps took 385 us; 16 tiles of 32 x 64 in 8 pieces occupy 128 SMs with 17 steps each (37 us).  Large
+// ones take tiles of 64 rows: 2048^3 506 us, with 32 rows 780, 655 before the pieces; 4096^2 with K = 16 28 us,
+// with full steps and scalar stores 56, before the pieces 32.
 #define GN 64
 #define GK 32
-template <bool TA, bool TB>
+template <int GM, bool TA, bool TB>
 __global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, int kc, const float* __restrict__ A, int lda,
                                                    const float* __restrict__ B, int ldb, float* __restrict__ C, int ldc,
                                                    float alpha, float beta, const GemmTail t)
@@ -64,11 +65,12 @@ __global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, int kc, 
     const int m0 = blockIdx.x * GM, n0 = blockIdx.y * GN;
     const int ka = blockIdx.z * kc, kb = min(K, ka + kc), nt = ka < kb ? (kb - ka + GK - 1) / GK : 0;
     const bool sums = t.bsum != nullptr && blockIdx.x == 0;
-    float acc[2][4] = {{0.f}}, bs = 0.f;
-    float ra[4], rb[8];
+    constexpr int GR = GM / 16;                  // rows of a thread
+    float acc[GR][4] = {{0.f}}, bs = 0.f;
+    float ra[GM / 8], rb[8];
     auto load = [&](int k0) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
+        for (int i = 0; i < GM / 8; i++) {
             const int e = tid + 256 * i;
             const int kk = TA ? e / GM : e % GK, mm = TA ? e % GM : e / GK;
             const int gm = m0 + mm, gk = k0 + kk;
@@ -84,7 +86,7 @@ __global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, int kc, 
     };
     auto put = [&](int u) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
+        for (int i = 0; i < GM / 8; i++) {
             const int e = tid + 256 * i;
             As[u][TA ? e / GM : e % GK][TA ? e % GM : e / GK] = ra[i];
         }
@@ -102,26 +104,58 @@ __global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, int kc, 
     for (int s = 0; s < nt; s++) {
         const int u = s & 1;
         if (s + 1 < nt) load(ka + (s + 1) * GK);
+        const int ke = kb - ka - s * GK;                 // (the last step: eight at a time)
 #pragma unroll
-        for (int kk = 0; kk < GK; kk++) {
-            const float a0 = As[u][kk][ty * 2], a1 = As[u][kk][ty * 2 + 1];
-            const float4 b = *reinterpret_cast<const float4*>(&Bs[u][kk][tx * 4]);
-            acc[0][0] = fmaf(a0, b.x, acc[0][0]); acc[0][1] = fmaf(a0, b.y, acc[0][1]);
-            acc[0][2] = fmaf(a0, b.z, acc[0][2]); acc[0][3] = fmaf(a0, b.w, acc[0][3]);
-            acc[1][0] = fmaf(a1, b.x, acc[1][0]); acc[1][1] = fmaf(a1, b.y, acc[1][1]);
-            acc[1][2] = fmaf(a1, b.z, acc[1][2]); acc[1][3] = fmaf(a1, b.w, acc[1][3]);
+        for (int k8 = 0; k8 < GK; k8 += 8) {
+            if (k8 >= ke) break;
+#pragma unroll
+            for (int kk = k8; kk < k8 + 8; kk++) {
+                const float4 b = *reinterpret_cast<const float4*>(&Bs[u][kk][tx * 4]);
+#pragma unroll
+                for (int i = 0; i < GR; i++) {
+                    const float a = As[u][kk][ty * GR + i];
+                    acc[i][0] = fmaf(a, b.x, acc[i][0]); acc[i][1] = fmaf(a, b.y, acc[i][1]);
+                    acc[i][2] = fmaf(a, b.z, acc[i][2]); acc[i][3] = fmaf(a, b.w, acc[i][3]);
+                }
+            }
         }
         if (sums && tid < GN)
             for (int kk = 0; kk < GK; kk++) bs += Bs[u][kk][tid];
         if (s + 1 < nt) put(u ^ 1);
         __syncthreads();
     }
+    auto out = [&](int gm, int gn, float v) {
+        if (gm >= M || gn >= N) return;
+        const size_t o = (size_t)gm * ldc + gn;
+        float z = alpha * v + (beta != 0.f ? beta * C[o] : 0.f);
+        if (t.bias) z += __ldg(&t.bias[gn]);
+        if (t.zgrad) z *= gelu_grad(__ldg(&t.zgrad[o]));
+        C[o] = z;
+        if (t.Y) t.Y[o] = t.act ? gelu(z) : z;
+    };
+    if (gridDim.z == 1) {                        // one piece: no tiles to add
+        const bool four = !t.bias && !t.zgrad && !t.Y && n0 + tx * 4 + 4 <= N && ldc % 4 == 0 && (reinterpret_cast<size_t>(C) & 15) == 0;
+#pragma unroll
+        for (int i = 0; i < GR; i++) {
+            const int gm = m0 + ty * GR + i;
+            if (four && beta == 0.f) {
+                if (gm < M)
+                    *reinterpret_cast<float4*>(&C[(size_t)gm * ldc + n0 + tx * 4]) =
+                        make_float4(alpha * acc[i][0], alpha * acc[i][1], alpha * acc[i][2], alpha * acc[i][3]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; j++) out(gm, n0 + tx * 4 + j, acc[i][j]);
+            }
+        }
+        if (sums && tid < GN && n0 + tid < N) t.bsum[n0 + tid] = bs;
+        return;
+    }
     // the piece's tile in shared memory (the operands are done with), then the sum over the cluster
     float* red = &Bs[0][0][0];
 #pragma unroll
-    for (int i = 0; i < 2; i++)
+    for (int i = 0; i < GR; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) red[(ty * 2 + i) * GN + tx * 4 + j] = acc[i][j];
+        for (int j = 0; j < 4; j++) red[(ty * GR + i) * GN + tx * 4 + j] = acc[i][j];
     if (sums && tid < GN) cs[tid] = bs;
     cg::cluster_group cl = cg::this_cluster();
     cl.sync();
@@ -129,14 +163,7 @@ __global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, int kc, 
     for (int e = r * 256 + tid; e < GM * GN; e += S * 256) {
         float v = 0.f;
         for (int q = 0; q < S; q++) v += *cl.map_shared_rank(red + e, q);
-        const int gm = m0 + e / GN, gn = n0 + e % GN;
-        if (gm >= M || gn >= N) continue;
-        const size_t o = (size_t)gm * ldc + gn;
-        float z = alpha * v + (beta != 0.f ? beta * C[o] : 0.f);
-        if (t.bias) z += __ldg(&t.bias[gn]);
-        if (t.zgrad) z *= gelu_grad(__ldg(&t.zgrad[o]));
-        C[o] = z;
-        if (t.Y) t.Y[o] = t.act ? gelu(z) : z;
+        out(m0 + e / GN, n0 + e % GN, v);
     }
     if (sums && r == 0 && tid < GN && n0 + tid < N) {
         float v = 0.f;
@@ -341,7 +368,12 @@ static int gemm(int M, int N, int K, const float* A, int lda, int transA, const 
         }
         return 0;
     }
-    const int tm = (M + GM - 1) / GM, tn = (N + GN - 1) / GN;
+    const int tn = (N + GN - 1) / GN;
+    // tiles of 64 rows (half the loads of B per multiplication) where they are many enough to fill the chip with
+    // pieces of K: 512 x 512, K = 512 (64 tiles) 21 us with 32 rows, 17 with 64; 256 x 256, K = 4109 (16 tiles)
+    // 37 and 46; 2000 x 64, K = 64 (32 tiles) 6 and 8.5
+    const int gm = (long long)((M + 63) / 64) * tn >= 64 ? 64 : 32;
+    const int tm = (M + gm - 1) / gm;
     // pieces of K: as many CTAs as two per SM, at least 64 steps of K each
     int S = 8;
     while (S > 1 && ((long long)tm * tn * S > 2 * 148 || K / S < 64)) S /= 2;
@@ -355,15 +387,12 @@ static int gemm(int M, int N, int K, const float* A, int lda, int transA, const 
     at.val.clusterDim.x = at.val.clusterDim.y = 1;
     at.val.clusterDim.z = S;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    cudaError_t e;
-    if (transA) {
-        if (transB) e = cudaLaunchKernelEx(&cfg, gemm_kernel<true, true>, M, N, K, kc, A, lda, B, ldb, C, ldc, alpha, beta, t);
-        else e = cudaLaunchKernelEx(&cfg, gemm_kernel<true, false>, M, N, K, kc, A, lda, B, ldb, C, ldc, alpha, beta, t);
-    } else {
-        if (transB) e = cudaLaunchKernelEx(&cfg, gemm_kernel<false, true>, M, N, K, kc, A, lda, B, ldb, C, ldc, alpha, beta, t);
-        else e = cudaLaunchKernelEx(&cfg, gemm_kernel<false, false>, M, N, K, kc, A, lda, B, ldb, C, ldc, alpha, beta, t);
-    }
+    cfg.numAttrs = S > 1 ? 1 : 0;
+    auto run = [&](auto k) { return cudaLaunchKernelEx(&cfg, k, M, N, K, kc, A, lda, B, ldb, C, ldc, alpha, beta, t); };
+    const cudaError_t e = gm == 64 ? (transA ? (transB ? run(gemm_kernel<64, true, true>) : run(gemm_kernel<64, true, false>))
+                                             : (transB ? run(gemm_kernel<64, false, true>) : run(gemm_kernel<64, false, false>)))
+                                   : (transA ? (transB ? run(gemm_kernel<32, true, true>) : run(gemm_kernel<32, true, false>))
+                                             : (transB ? run(gemm_kernel<32, false, true>) : run(gemm_kernel<32, false, false>)));
     return launch_status(e);
 }
 
