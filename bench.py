@@ -340,13 +340,6 @@ def run_reference(args, rank, world):
 # ------------------------------------------------------------------------------------------------
 # our arm
 # ------------------------------------------------------------------------------------------------
-def kernel_bytes(k):
-    """Algorithmic bytes of one pass (both components, read + write, complex FP32)."""
-    if k[0] == 'resize':
-        return 2 * 8 * (k[1] * k[2] + k[3] * k[4])
-    return 2 * 8 * 2 * k[1] * k[2]
-
-
 def hbm_peak():
     """(HBM GB/s, 'measured' | 'fallback'): the measured copy bandwidth of this GPU pool when the
     peaks file is present, else the earlier measured fallback figure."""
@@ -364,38 +357,35 @@ def sampled_rows(acc, out):
     return len(np.union1d(i, i + 1))
 
 
-def batch_bytes(me, nb, out):
-    """Algorithmic bytes of every pass of a launch of nb electrons of `me` (MultiE) from its shapes: what a pass
-    reads and writes of both components, windows only where passes leave out what is zero (the planner's
-    description of the base electron), the base field read once; a last pass that writes the intensity one
-    float per point, one that reads sampled rows only those (and so the column pass before it writes only
-    those) and the detector's FP64 sums once."""
-    lines = [l for l in me.describe().splitlines() if l.split()[1] in ('LINE', 'RESIZE')]
-    win = lambda l: [int(v) for p in re.findall(r'(?:lines=|points=)(-?\d+):(-?\d+)', l) for v in p]  # noqa: E731
-    step = (me._accm.yFin - me._accm.yStart) / (me.ny - 1)
-    rows = sampled_rows(me._accm, out)
+def shape_bytes(text, nb=1, rows=None, det=None):
+    """Algorithmic bytes of the line and resize passes of a launch of nb wavefronts from the planner's
+    description: what a pass reads and writes of both components, windows only where passes leave out what is
+    zero (the base wavefront's), the input field once; a last pass that writes the intensity one float per
+    point; with `rows` the last row pass reads only that many (and the column pass before it writes only
+    those) and the sums of `det` detector points once."""
+    lines = [l for l in text.splitlines() if l.split()[1] in ('LINE', 'RESIZE')]
     res = []
     for i, l in enumerate(lines):
         f = l.split()
         if f[1] == 'RESIZE':
             nxo, nzo = map(int, f[2].split('x'))
+            nxn, nzn = map(int, f[4].split('x'))
             x0, x1, z0, z1 = map(int, re.search(r'window=x(-?\d+):(-?\d+),z(-?\d+):(-?\d+)', l).groups())
-            res.append(16 * nxo * nzo + nb * 16 * (x1 - x0 + 1) * (z1 - z0 + 1))
+            zero = i + 1 == len(lines) or 'zwin=0' in lines[i + 1]          # zeros around the window are written
+            res.append(16 * nxo * nzo + nb * 16 * (nxn * nzn if zero else (x1 - x0 + 1) * (z1 - z0 + 1)))
             continue
         nx, nz = map(int, f[3].split('x'))
         N, nl = (nx, nz) if f[2] == 'rows' else (nz, nx)
-        w = win(l)
+        w = [int(v) for p in re.findall(r'(?:lines=|points=)(-?\d+):(-?\d+)', l) for v in p]
         wl, wp = (w[1] - w[0] + 1, w[3] - w[2] + 1) if w else (nl, N)
         last = i + 1 == len(lines)
-        sampled = lambda q: ('intensity' in q and ' LINE rows' in q and  # noqa: E731
-                             step >= 2. * abs(out['yFin'] - out['yStart']) / (out['ny'] - 1))
-        read = 16 * wl * wp if i else 16 * wl * wp / nb
-        write = 16 * wl * N
+        read = 16 * wl * wp if i else 16. * wl * wp / nb
+        write = 16 * (nl if last else wl) * N
         if last and 'intensity' in l:
             write = 4 * nl * N
-            if sampled(l):
-                read, write = 16 * rows * wp, 8. * me.nx * me.ny / nb
-        elif not last and sampled(lines[i + 1]) and f[2] == 'cols':
+            if rows:
+                read, write = 16 * rows * wp, 8. * det / nb
+        elif rows and i + 2 == len(lines):
             write = 16 * wl * rows
         res.append(nb * (read + write))
     return res
@@ -404,12 +394,15 @@ def batch_bytes(me, nb, out):
 def batched_passes(me, offs, stream, peak, peak_src, where, out):
     """One batch of the multi-electron object `me` (MultiE, output mesh `out`) run without its graph, with CUDA
     events around every pass (srwgMultiEAddTimed; adds the electrons): per-pass times and the roofline of the
-    dominant pass, algorithmic bytes (batch_bytes) over the pass's CUDA-event time."""
+    dominant pass, algorithmic bytes (shape_bytes) over the pass's CUDA-event time."""
     ks, inten = me.info()
     ms = me.add_timed(offs, stream)
     nb = len(offs)
     per = ms[:len(ks)]
-    alg = batch_bytes(me, nb, out)
+    m = me._accm
+    sampled = (ks[-1][0] == 'line_rows' and inten and
+               (m.yFin - m.yStart) / (m.ny - 1) >= 2. * abs(out['yFin'] - out['yStart']) / (out['ny'] - 1))
+    alg = shape_bytes(me.describe(), nb, sampled_rows(m, out) if sampled else None, me.nx * me.ny)
     kd = int(np.argmax(per))
     achieved = alg[kd] / (per[kd] / 1000.) / 1e9
     return {"bound": "hbm", "kernel": "%s %s (batch of %d)" % (ks[kd][0], 'x'.join(map(str, ks[kd][1:])), nb),
@@ -864,7 +857,7 @@ def run_ours(args, rank, world):
                                           "passes": [list(k) for k in pl_l['kinfo']],
                                           "per_pass_ms": [round(float(v), 4) for v in pl_l['per_k']]}
     peak, peak_src = hbm_peak()
-    pass_bytes = sum(kernel_bytes(k) for k in kinfo)
+    pass_bytes = int(sum(shape_bytes(plan.describe())))
     # algorithmic bytes of one propagation (model: resize reads the old and writes the new mesh,
     # one 2D FFT = one read + one write pass per axis at the new mesh, point-wise work fused; both
     # components): [8 N_in + 8 N_out + 2 * 16 N_out] * 2 = 1,358,954,496 B for 1024^2 -> 4096^2
@@ -960,7 +953,7 @@ def roofline(pl, peak, peak_src, where):
     over its average CUDA-event time, against the HBM peak."""
     kinfo, per_k = pl['kinfo'], pl['per_k']
     kd = int(np.argmax(per_k))
-    alg = kernel_bytes(kinfo[kd])
+    alg = int(shape_bytes(pl['plan'].describe())[kd])
     achieved = alg / (per_k[kd] / 1000.) / 1e9
     return {"bound": "hbm", "kernel": "%s %s" % (kinfo[kd][0], 'x'.join(map(str, kinfo[kd][1:]))),
             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_src,
