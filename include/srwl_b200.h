@@ -310,17 +310,18 @@ SRWG_API int srwgPropagElecFieldStatic(const SRWLWfr* pWfr, const SRWLOptC* pOpt
                                        const float* dEyIn, float* dExOut, float* dEyOut, long long outCapacity,
                                        void* stream, SRWLWfr* pWfrOut);
 
-/* Autotuned launch shapes (no counterpart in the reference, whose FFTs are FFTW's): kernel family
- * (1: the power-of-two pass, 3: the specialised pass of linen_lengths.h, which also serves the powers
- * of two listed there) and lines per CTA of the line passes with compile-time lengths, per axis
- * (0 rows, 1 columns) and line length N.  The library reads the table measured by srw_b200.tune from
+/* Autotuned launch shapes (no counterpart in the reference, whose FFTs are FFTW's): lines per CTA of
+ * the line passes of the tuned lengths (two lines a pair: odd numbers launch one line less, at least
+ * two), per axis (0 rows, 1 columns) and length N.  A length's family (1: powers of two, 3: the general
+ * lengths of linen_lengths.h, and the powers of two listed there on request) bounds the lines an entry
+ * may have; it chooses no kernel.  The library reads the table measured by srw_b200.tune from
  * models/line_tuning.txt beside its directory (or the file named by the environment variable
- * SRWG_TUNING; "" for the built-in defaults) at its first plan.
- *   srwgTuneSetFamily: sets the family of one entry (0: the length's default); error 23903 when the
- *                      family has no kernel for N
+ * SRWG_TUNING; "" for the built-in choice) at its first plan.
+ *   srwgTuneSetFamily: sets the family of one entry (0: the length's own); error 23903 when N is
+ *                      not of that family
  *   srwgTuneSetLines:  sets the lines per CTA of one entry in its family (0 removes the entry);
  *                      error 23903 for an invalid shape
- *   srwgTuneGetFamily / srwgTuneGetLines: what plans use now (0: not a compile-time length)
+ *   srwgTuneGetFamily / srwgTuneGetLines: what plans use now (0: not a tuned length)
  *   srwgTuneLoad:      replaces the table by a file's entries (NULL or "": defaults only) */
 SRWG_API int srwgTuneSetFamily(int axis, int N, int family);
 SRWG_API int srwgTuneSetLines(int axis, int N, int lines);
@@ -328,7 +329,7 @@ SRWG_API int srwgTuneGetFamily(int axis, int N, int* family);
 SRWG_API int srwgTuneGetLines(int axis, int N, int* lines);
 SRWG_API int srwgTuneLoad(const char* path, int* nEntries);
 
-/* Bounded waits of the kernels (the specialised line passes wait for the bulk copies of their input
+/* Bounded waits of the kernels (line passes wait for the bulk copies of their input
  * tiles): srwgSetWaitLimit sets the iteration limit of those waits (0: the built-in limit, far above
  * any copy's time); a wait that reaches it counts the event in a per-device counter, lets the copies
  * in flight land, and the CTA skips its work (the pass's output is then incomplete).

@@ -146,9 +146,8 @@ static double flat_mag2(const std::vector<float2>& T, long long off, int n)
     return (hi > 0. && hi - lo <= 1e-6 * hi) ? 0.5 * (lo + hi) : -1.;
 }
 
-// the last pass writes the total intensity instead of the two fields where it runs on a specialised
-// kernel with one transform and no non-separable work (the accumulation then reads one float per
-// sample instead of two complex values).  Where its output factors -- the output chain's table along
+// the last pass writes the total intensity instead of the two fields where it runs on pairs with one transform
+// and no non-separable work (the accumulation then reads one float per sample instead of two complex values).  Where its output factors -- the output chain's table along
 // the lines and every chain's line factor -- have one magnitude, |f v|^2 = |f|^2 |v|^2: the pass
 // skips them and scales the intensity by that magnitude squared.
 // Along the rows of a run with sampled rows (sampled_rows), only the two rows around each detector row (anx

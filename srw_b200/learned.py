@@ -400,7 +400,9 @@ def factor_error(I, om, I_ref, om_ref, box):
 
 
 # ------------------------------------------------------------------------------------------------
-# cost model: autotuned per-length pass times (srw_b200.tune), per point
+# cost model: per-length pass times (models/line_tuning.json), per point.  They were measured on the one-line passes
+# that came before those on pairs; the ratios between lengths choose the factors, and the network was evaluated
+# with these choices.
 # ------------------------------------------------------------------------------------------------
 _TIMES = None
 
@@ -425,12 +427,12 @@ FILLED = 1024            # shortest line length whose single-wavefront passes fi
 
 
 def point_costs(n):
-    """(row, column) pass time per point [ms] of length n from the tuning table.  The table times
+    """(row, column) pass time per point [ms] of length n from the table of times.  The table times
     one wavefront; below FILLED points per line its passes are too small to fill the GPU and the
     time is mostly launch and tail latency, which a batch of wavefronts does not pay per wavefront,
     so there the per-point time of the shortest measured length from FILLED up of the same kind
     (power of two or not) stands in.  A length the table lacks gets the largest per-point time of
-    its measured neighbours times 3 (the run-time-scheduled kernel)."""
+    its measured neighbours times 3 (what such lengths took then)."""
     t = _times()
     if not t:
         return (1., 1.) if (n & (n - 1)) == 0 else (5., 5.)
