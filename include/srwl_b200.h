@@ -204,7 +204,10 @@ SRWG_API int srwgPlanInfo(const srwgPlan* plan, long* nxIn, long* nyIn, long* nx
 
 /* Executes the plan on device arrays (interleaved complex FP32, [ny][nx]) on CUDA stream
  * `stream` (NULL = default stream).  dExIn/dEyIn are read only; the result (output mesh) is
- * written to dExOut/dEyOut, which must hold nxOut*nyOut complex values each. */
+ * written to dExOut/dEyOut, which must hold nxOut*nyOut complex values each.  Executions of all plans of
+ * a device share its work buffers: on different streams they run one after the other, in the order of
+ * the calls.  A graph captured from an execution names those buffers: order its replays with other
+ * executions, and keep them from growing (a plan of a larger grid makes new ones). */
 SRWG_API int srwgPlanExecute(srwgPlan* plan, const float* dExIn, const float* dEyIn, float* dExOut, float* dEyOut,
                     void* stream);
 

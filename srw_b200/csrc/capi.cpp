@@ -449,6 +449,35 @@ static int ensure_doubles(double** buf, size_t* cap, size_t n)
 
 // runs the plan's passes on one wavefront (or nb wavefronts with the same plan); moment passes
 // write their sums to momSlots (nMomSlots * SRWG_MOM_SLOT doubles per wavefront)
+// All plans of a device share its work buffers, on whatever streams they run.  While one stream uses them its order
+// is enough; from the second one on an execution waits on its stream for the one queued before it, which recorded
+// the event when it was queued (both take 1 us of host time, 4 % of a propagation at
+// 64 x 64, which programs of one stream don't pay).  A stream under capture takes part in neither: its graph's
+// replays are ordered by who launches them.
+static int work_begin(DeviceCtx& c, cudaStream_t st, bool* record)
+{
+    *record = false;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone ||
+        (c.workDone == nullptr && cudaStreamGetId(st, &id) != cudaSuccess)) {
+        cudaGetLastError();
+        return 0;
+    }
+    if (c.workDone != nullptr) {
+        CUDA_TRY(cudaStreamWaitEvent(st, c.workDone, 0));
+    } else if (c.workStream == 0 || c.workStream == id) {
+        c.workStream = id;
+        return 0;
+    } else {
+        // the first stream's executions recorded nothing (and it may be gone): wait for the device once
+        CUDA_TRY(cudaEventCreateWithFlags(&c.workDone, cudaEventDisableTiming));
+        if (cudaDeviceSynchronize() != cudaSuccess) cudaGetLastError();      // (refused while some stream is under capture)
+    }
+    *record = true;
+    return 0;
+}
+
 static int execute(Planner& pl, DeviceCtx& c, const float2* inX, const float2* inY, float2* outX, float2* outY,
                    float2* work, size_t workElems, const float2* dtab, cudaStream_t st, cudaEvent_t* ev = nullptr,
                    int nb = 1, long long inStride = 0, long long outStride = 0, double* momSlots = nullptr,
@@ -468,8 +497,13 @@ static int execute(Planner& pl, DeviceCtx& c, const float2* inX, const float2* i
     }
     size_t descOff;
     const_bytes(pl, &descOff);
-    return execute_passes(pl.kernels, c, nb, inX, inY, inStride, outX, outY, outStride, work, workElems,
-                          (const char*)dtab, 0, descOff, st, ev, nullptr, momScratch, momSlots, pl.nMomSlots, intOut);
+    bool record;
+    int r = work_begin(c, st, &record);
+    if (r) return r;
+    r = execute_passes(pl.kernels, c, nb, inX, inY, inStride, outX, outY, outStride, work, workElems,
+                       (const char*)dtab, 0, descOff, st, ev, nullptr, momScratch, momSlots, pl.nMomSlots, intOut);
+    if (record) CUDA_TRY(cudaEventRecord(c.workDone, st));
+    return r;
 }
 
 static int ensure_work(DeviceCtx& c, size_t elems)

@@ -14,6 +14,8 @@ struct DeviceCtx {
     std::map<int, float2*> tw;          // twiddle tables by FFT length
     float2* work = nullptr;             // 2 work buffers x 2 components
     size_t workElems = 0;               // per buffer per component
+    unsigned long long workStream = 0;  // the stream that used them (its id; 0: none yet), while there is only one
+    cudaEvent_t workDone = nullptr;     // from the second stream on: the last execution has finished
     float2* io = nullptr;               // input + output staging for the host-memory entry point
     size_t ioElems = 0;
     float2* tab = nullptr;              // point-wise tables of the one-shot entry point
