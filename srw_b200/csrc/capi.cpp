@@ -451,9 +451,10 @@ static int ensure_doubles(double** buf, size_t* cap, size_t n)
 // write their sums to momSlots (nMomSlots * SRWG_MOM_SLOT doubles per wavefront)
 // All plans of a device share its work buffers, on whatever streams they run.  While one stream uses them its order
 // is enough; from the second one on an execution waits on its stream for the one queued before it, which recorded
-// the event when it was queued (both take 1 us of host time, 4 % of a propagation at
-// 64 x 64, which programs of one stream don't pay).  A stream under capture takes part in neither: its graph's
-// replays are ordered by who launches them.
+// the event when it was queued (both take 1 us of host time, 5 % of a propagation at 64 x 64, which programs of
+// one stream don't pay).  The library's own stream (calls on host memory) has finished when its call returns: it
+// waits for the others and nobody for it.  A stream under capture takes no part: its graph's replays are
+// ordered by who launches them.
 static int work_begin(DeviceCtx& c, cudaStream_t st, bool* record)
 {
     *record = false;
@@ -464,17 +465,22 @@ static int work_begin(DeviceCtx& c, cudaStream_t st, bool* record)
         cudaGetLastError();
         return 0;
     }
+    const bool own = st == c.stream;
     if (c.workDone != nullptr) {
         CUDA_TRY(cudaStreamWaitEvent(st, c.workDone, 0));
-    } else if (c.workStream == 0 || c.workStream == id) {
-        c.workStream = id;
+        *record = true;
         return 0;
-    } else {
-        // the first stream's executions recorded nothing (and it may be gone): wait for the device once
-        CUDA_TRY(cudaEventCreateWithFlags(&c.workDone, cudaEventDisableTiming));
-        if (cudaDeviceSynchronize() != cudaSuccess) cudaGetLastError();      // (refused while some stream is under capture)
     }
-    *record = true;
+    if (c.workStream != 0 && c.workStream != id) {
+        // the first stream's executions recorded nothing (and it may be gone): wait for the device once
+        // (refused while some stream is under capture)
+        if (cudaDeviceSynchronize() != cudaSuccess) cudaGetLastError();
+        if (!own) {
+            CUDA_TRY(cudaEventCreateWithFlags(&c.workDone, cudaEventDisableTiming));
+            *record = true;
+        }
+    }
+    c.workStream = own ? 0 : id;
     return 0;
 }
 
