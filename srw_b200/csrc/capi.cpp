@@ -451,8 +451,8 @@ static int ensure_doubles(double** buf, size_t* cap, size_t n)
 // write their sums to momSlots (nMomSlots * SRWG_MOM_SLOT doubles per wavefront)
 // All plans of a device share its work buffers, on whatever streams they run.  While one stream uses them its order
 // is enough; from the second one on an execution waits on its stream for the one queued before it, which recorded
-// the event when it was queued (both take 1 us of host time, 5 % of a propagation at 64 x 64, which programs of
-// one stream don't pay).  The library's own stream (calls on host memory) has finished when its call returns: it
+// the event when it was queued (0.35 us of host time on the default stream; the checks 0.1 us; a propagation at
+// 64 x 64 takes 20).  The library's own stream (calls on host memory) has finished when its call returns: it
 // waits for the others and nobody for it.  A stream under capture takes no part: its graph's replays are
 // ordered by who launches them.
 static int work_begin(DeviceCtx& c, cudaStream_t st, bool* record)
