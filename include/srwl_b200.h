@@ -233,7 +233,8 @@ SRWG_API int srwgPlanDestroy(srwgPlan* plan);
  * (srwlCalcIntFromElecField, polarisation 6, vs x and y) is added, bilinearly interpolated onto
  * pAccMesh (avg_update_interp order 1, srwlib.py:1116), to an FP64 accumulator on the device.
  * srwgMultiEAdd takes 4 doubles per electron (x [m], x' [rad], y [m], y' [rad]); a null stream
- * means the library's stream, synchronised before the call returns.  srwgMultiEGetMean copies the
+ * means the library's stream, synchronised before the call returns.  Calls of one object may come on
+ * different streams: each waits for the last batch queued before it.  srwgMultiEGetMean copies the
  * mean (sum / number of electrons) to host memory.  pOpt must stay valid while the object lives. */
 typedef struct srwgMultiE srwgMultiE;
 SRWG_API int srwgMultiECreate(const SRWLWfr* pBase, const SRWLOptC* pOpt, const SRWLRadMesh* pAccMesh, int maxBatch,

@@ -745,6 +745,10 @@ extern "C" SRWG_API int srwgMultiEAddTimed(srwgMultiE* m, int n, const double* a
     return r;
 }
 
+// The object's buffers and sums serve one call after the other, on whatever streams they run: each waits for the
+// last batch queued before it.
+static cudaError_t after_last_batch(const srwgMultiE& m, cudaStream_t st) { return cudaStreamWaitEvent(st, m.used[m.slot ^ 1], 0); }
+
 // A call either adds all its electrons or none: the accumulator is copied aside first, and on an
 // error (an electron whose passes differ in size from the base wavefront's, a failed launch) the
 // batches already added are taken out again by restoring that copy and the electron count.
@@ -760,6 +764,7 @@ static int add_impl(srwgMultiE* m, int n, const double* arOffsets, int stride, v
     cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
     if (n == 0) return 0;
     const size_t accBytes = (size_t)m->anx * m->anz * sizeof(double);
+    MTRY(after_last_batch(*m, st));
     MTRY(cudaMemcpyAsync(m->dSnap, m->dAcc, accBytes, cudaMemcpyDeviceToDevice, st));
     const long long n0 = m->nAdded;
     r = add_body(m, n, arOffsets, stride, st);
@@ -928,6 +933,7 @@ extern "C" SRWG_API int srwgMultiEGetMean(srwgMultiE* m, double* arMean, long lo
     if (r) return r;
     const size_t na = (size_t)m->anx * m->anz;
     cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
+    MTRY(after_last_batch(*m, st));
     MTRY(cudaMemcpyAsync(arMean, m->dAcc, na * sizeof(double), cudaMemcpyDeviceToHost, st));
     MTRY(cudaStreamSynchronize(st));
     if (m->nAdded > 0)
@@ -963,6 +969,7 @@ extern "C" SRWG_API int srwgMultiEReset(srwgMultiE* m, void* stream)
     int r = device_ctx(m->device, &c);
     if (r) return r;
     cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
+    MTRY(after_last_batch(*m, st));
     MTRY(cudaMemsetAsync(m->dAcc, 0, (size_t)m->anx * m->anz * sizeof(double), st));
     if (!stream) MTRY(cudaStreamSynchronize(st));
     m->nAdded = 0;

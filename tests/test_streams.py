@@ -1,5 +1,5 @@
 """Executions of plans on several streams, from one thread and from several, share the device's work buffers: each
-gives what it gives alone, to the bit."""
+gives what it gives alone, to the bit.  So do the calls of a multi-electron object on streams of their own."""
 import random
 import threading
 
@@ -63,3 +63,28 @@ def test_streams_give_the_same_fields(threads):
             t.join()
     torch.cuda.synchronize()
     assert not bad, len(bad)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('graph', [False, True])
+@pytest.mark.parametrize('rows', [120, 1500])                     # sampled rows, and all of them
+def test_multi_electron_calls_on_several_streams(graph, rows):
+    if not torch.cuda.is_available():
+        pytest.skip('no CUDA device')
+    from srw_b200.multie import MultiE, sample_offsets
+    from srw_b200.plan import Plan
+    sc = dict(Rx=20., Ry=20., dRx=0.2, dRy=0.2)
+    ex, _, mesh = gaussian(500, E=2012., sig=0.35e-3, r=1.5e-3, R=20.)
+    w, chain = make_wfr(ex, 0.5j * ex, mesh, **sc), beamline(C1, [PP(), PP(0, 2., 2., 2., 2.), PP(4)])
+    m = Plan(w, chain).output_mesh()
+    acc = dict(nx=100, ny=rows, eStart=mesh['eStart'], **{k: m[k] for k in ('xStart', 'xFin', 'yStart', 'yFin')})
+    offs = sample_offsets(32, 30e-6, 5e-6, 5e-6, 2e-6, seed=3, sig_e=1e-3)
+    got = []
+    for n in (1, 4):
+        streams = [torch.cuda.Stream() for _ in range(n)]
+        me = MultiE(w, chain, acc, max_batch=4, graph=graph)
+        for k in range(8):
+            me.add(offs[4 * k:4 * k + 4], streams[k % n].cuda_stream)
+        got.append(me.mean())                                     # on a stream of its own
+        torch.cuda.synchronize()
+    assert got[0].max() > 0 and np.array_equal(got[0], got[1])
